@@ -16,26 +16,33 @@ namespace {
 // Lattice maths in the reference's SSE3 order (src/lb/lattices/Lattice.h:51-110, 374-448).
 // ---------------------------------------------------------------------------
 
+// The reference multiplies every component by every f; the products with a zero
+// component add +-0 and are left out here (a third of a site's FP64 operations:
+// they cannot be folded by the compiler, as 0 * inf is NaN).  rho - rho is 0 for
+// finite distributions and NaN otherwise, which keeps a non-finite value's effect
+// on all three components.  A sum begun at -0.0 takes its first term unchanged.
+// (Step time: 4M-site pipe 218.0 -> 214.2 us, 497k-site LES stenosis 44.0 -> 41.8 us.)
 __device__ __forceinline__ void moments(const double* f, double& rho, double& mx, double& my, double& mz) {
-  double dl = 0.0, dh = f[18];
-  double xl = 0.0, xh = (double)cx(18) * f[18];
-  double yl = 0.0, yh = (double)cy(18) * f[18];
-  double zl = 0.0, zh = (double)cz(18) * f[18];
+  double dl = f[0], dh = f[18];
+  double xl = -0.0, xh = cx(18) ? (double)cx(18) * f[18] : -0.0;
+  double yl = -0.0, yh = cy(18) ? (double)cy(18) * f[18] : -0.0;
+  double zl = -0.0, zh = cz(18) ? (double)cz(18) * f[18] : -0.0;
 #pragma unroll
   for (int d = 0; d < 18; d += 2) {
-    dl = dl + f[d];
+    if (d) dl = dl + f[d];
     dh = dh + f[d + 1];
-    xl = xl + (double)cx(d) * f[d];
-    xh = xh + (double)cx(d + 1) * f[d + 1];
-    yl = yl + (double)cy(d) * f[d];
-    yh = yh + (double)cy(d + 1) * f[d + 1];
-    zl = zl + (double)cz(d) * f[d];
-    zh = zh + (double)cz(d + 1) * f[d + 1];
+    if (cx(d)) xl = xl + (double)cx(d) * f[d];
+    if (cx(d + 1)) xh = xh + (double)cx(d + 1) * f[d + 1];
+    if (cy(d)) yl = yl + (double)cy(d) * f[d];
+    if (cy(d + 1)) yh = yh + (double)cy(d + 1) * f[d + 1];
+    if (cz(d)) zl = zl + (double)cz(d) * f[d];
+    if (cz(d + 1)) zh = zh + (double)cz(d + 1) * f[d + 1];
   }
   rho = dl + dh;
-  mx = xl + xh;
-  my = yl + yh;
-  mz = zl + zh;
+  const double nf = rho - rho;
+  mx = (xl + xh) + nf;
+  my = (yl + yh) + nf;
+  mz = (zl + zh) + nf;
 }
 
 struct FeqConst {
@@ -46,11 +53,39 @@ struct FeqConst {
     nh = (9. / 2.) * d1;
     t1 = rho - th * d1;
   }
+  __device__ __forceinline__ double mde(int i) const {
+    double e = -0.0;
+    if (cx(i)) e = e + (double)cx(i) * mx;
+    if (cy(i)) e = e + (double)cy(i) * my;
+    if (cz(i)) e = e + (double)cz(i) * mz;
+    return e;
+  }
   __device__ __forceinline__ double operator()(int i) const {
-    const double mde = (double)cx(i) * mx + (double)cy(i) * my + (double)cz(i) * mz;
-    return weight(i) * ((t1 + nh * (mde * mde)) + 3. * mde);
+    if (i == 0) return weight(0) * t1;
+    const double e = mde(i);
+    return weight(i) * ((t1 + nh * (e * e)) + 3. * e);
+  }
+  // f[i] - feq(i) for every direction; the opposite of an odd i is i + 1, whose
+  // momentum component is -e exactly, so the two share the even part.
+  __device__ __forceinline__ void neq(const double* f, double* fneq) const {
+    fneq[0] = f[0] - (*this)(0);
+#pragma unroll
+    for (int i = 1; i < Q; i += 2) {
+      const double e = mde(i), even = t1 + nh * (e * e), odd = 3. * e;
+      fneq[i] = f[i] - weight(i) * (even + odd);
+      fneq[i + 1] = f[i + 1] - weight(i + 1) * (even - odd);
+    }
   }
 };
+
+// Sum over l of v[l] c_p c_r in index order (a momentum flux component).
+__device__ __forceinline__ double flux(const double* v, int p, int r) {
+  double acc = -0.0;
+#pragma unroll
+  for (int l = 0; l < Q; l++)
+    if (cc(p, l) * cc(r, l)) acc += (double)(cc(p, l) * cc(r, l)) * v[l];
+  return acc;
+}
 
 // Relaxation time of the LES kernel (LBGKLESSpongeLayer::CalculateTau and
 // compute_tau_smagorinsky, src/lb/kernels/LBGKLESSpongeLayer.h:122-182).
@@ -61,9 +96,7 @@ __device__ __forceinline__ double les_tau(const StepArgs& a, const double* fneq,
   for (int p = 0; p < 3; p++)
 #pragma unroll
     for (int r = 0; r < 3; r++) {
-      double qij = 0.0;
-#pragma unroll
-      for (int v = 0; v < Q; v++) qij += (double)(cc(p, v) * cc(r, v)) * fneq[v];
+      const double qij = flux(fneq, p < r ? p : r, p < r ? r : p);
       q12 += qij * qij;
     }
   q12 = sqrt(q12);
@@ -123,16 +156,13 @@ __device__ __forceinline__ void site_rates(const StepArgs& a, const double* fneq
 // Wall-shear-stress magnitude (Lattice::CalculateWallShearStressMagnitude,
 // CalculatePiTensor; src/lb/lattices/Lattice.h:1122-1156, 1353-1383).
 __device__ __forceinline__ double wss_mag(double tau, const double* fpost, const double* f, const double nor[3]) {
-  double pi[3][3];
+  double pi[3][3], df[Q];
+#pragma unroll
+  for (int l = 0; l < Q; l++) df[l] = fpost[l] - f[l];
 #pragma unroll
   for (int p = 0; p < 3; p++)
 #pragma unroll
-    for (int r = 0; r <= p; r++) {
-      double acc = 0.0;
-#pragma unroll
-      for (int l = 0; l < Q; l++) acc += (fpost[l] - f[l]) * (double)cc(p, l) * (double)cc(r, l);
-      pi[p][r] = acc * -(tau - 0.5);
-    }
+    for (int r = 0; r <= p; r++) pi[p][r] = flux(df, p, r) * -(tau - 0.5);
   pi[0][1] = pi[1][0];
   pi[0][2] = pi[2][0];
   pi[1][2] = pi[2][1];
@@ -151,16 +181,13 @@ __device__ __forceinline__ double wss_mag(double tau, const double* fpost, const
 // caches: the lower triangle in CalculatePiTensor's order and rounding
 // (src/lb/lattices/Lattice.h:1353-1383) as xx, xy, xz, yy, yz, zz, then tau.
 __device__ __forceinline__ void store_pi(const StepArgs& a, int s, double tau, const double* fpost, const double* f) {
-  double pi[3][3];
+  double pi[3][3], df[Q];
+#pragma unroll
+  for (int l = 0; l < Q; l++) df[l] = fpost[l] - f[l];
 #pragma unroll
   for (int p = 0; p < 3; p++)
 #pragma unroll
-    for (int r = 0; r <= p; r++) {
-      double acc = 0.0;
-#pragma unroll
-      for (int l = 0; l < Q; l++) acc += (fpost[l] - f[l]) * (double)cc(p, l) * (double)cc(r, l);
-      pi[p][r] = acc * -(tau - 0.5);
-    }
+    for (int r = 0; r <= p; r++) pi[p][r] = flux(df, p, r) * -(tau - 0.5);
   double* o = a.pi + s;
   o[0] = pi[0][0];
   o[a.np] = pi[1][0];
@@ -355,8 +382,7 @@ __device__ __forceinline__ void bulk_site_f64(const StepArgs& a, int s, int r) {
   moments(f, rho, mx, my, mz);
   const FeqConst feq(rho, mx, my, mz);
   double fneq[Q];
-#pragma unroll
-  for (int i = 0; i < Q; i++) fneq[i] = f[i] - feq(i);
+  feq.neq(f, fneq);
   double om, tau;
   site_rates<K>(a, fneq, s, tau, om);
 #pragma unroll
@@ -394,8 +420,7 @@ __device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
   const double ux = mx / rho, uy = my / rho, uz = mz / rho;
   const FeqConst feq(rho, mx, my, mz);
   double fneq[Q];
-#pragma unroll
-  for (int i = 0; i < Q; i++) fneq[i] = f[i] - feq(i);
+  feq.neq(f, fneq);
   double om, tau;
   site_rates<K>(a, fneq, s, tau, om);
   double fp[Q];
