@@ -59,6 +59,7 @@ struct GeneralDev {
   const int* io;          // [G] iolet table index or -1
   const int* cpl;         // [G] Windkessel coupling slot or -1
   const int* xyz;         // [3][G] global coordinates
+  const uint32_t* gzs;    // [G] wall links whose value the GZS link list computes (GZS walls only)
   const int* wom;         // [G] row of a Womersley iolet site in StepArgs::wom_amp, or -1 (null without one)
 };
 
@@ -73,6 +74,11 @@ struct StepArgs {
   const int* run_off;
   const int* run_po;      // [runs][20] plane offsets i * np + run_off[run][i] (shifted forms' bulk kernel), or null
   GeneralDev gen;
+  // GZS wall links with a virtual node (GZS walls only): the record and the
+  // direction of each, 32 records' links of one direction after the other.
+  const int* gzs_rec;
+  const uint8_t* gzs_dir;
+  int gzs_n;
   // kernel parameters
   double tau, omega, omega_minus;
   double lambda;          // TRT magic parameter (TRTSL: per-site omega_minus)

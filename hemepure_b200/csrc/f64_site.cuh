@@ -257,18 +257,6 @@ __device__ __forceinline__ bool link_velocity(const StepArgs& a, const IoletDev&
 
 __device__ __forceinline__ double ld(const double* p) { return __ldg(p); }
 
-// Pre-collision f of a plain bulk site.
-__device__ __forceinline__ void load_run_offsets(const StepArgs& a, int r, int* off);
-
-__device__ __forceinline__ void gather_bulk(const StepArgs& a, int s, int r, double* f) {
-  int off[20];
-  load_run_offsets(a, r, off);
-  f[0] = ld(a.fin + s);
-#pragma unroll
-  for (int i = 1; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + (s + off[i]));
-}
-
-// Pre-collision f of general site g (rules above).
 __device__ __forceinline__ void load_run_offsets(const StepArgs& a, int r, int* off) {
   const int4* o4 = reinterpret_cast<const int4*>(a.run_off) + 5 * r;
 #pragma unroll
@@ -281,31 +269,40 @@ __device__ __forceinline__ void load_run_offsets(const StepArgs& a, int r, int* 
   }
 }
 
+// Link masks and run of a site: a general record's own, none for a plain bulk site.
+struct Links {
+  uint32_t wall, iolet;
+  int run, g;
+};
+
+// The source of every slot i of site s before any boundary rule: s + run_off[run][i]
+// for a site whose bulk slots follow its run (L1-resident offsets), else the
+// record's pull table entry (which holds the record's own site for a slot that a
+// boundary rule fills).
+__device__ __forceinline__ void load_sources(const StepArgs& a, const Links& l, int s, int* src) {
+  if (l.run >= 0) {
+    int off[20];
+    load_run_offsets(a, l.run, off);
+#pragma unroll
+    for (int i = 1; i < Q; i++) src[i - 1] = s + off[i];
+  } else {
+#pragma unroll
+    for (int i = 1; i < Q; i++) src[i - 1] = __ldg(a.gen.src + (int64_t)(i - 1) * a.gen.G + l.g);
+  }
+}
+
 // Every slot's first value is one load whose address needs no branch: the
 // ghost of an iolet link, f*_d of the own site for a wall link, f*_i of the
-// source site otherwise.  The source site of slot i is s + run_off[run][i] for a
-// record whose bulk slots follow its run (L1-resident offsets), else the
-// record's pull table entry (which holds the record's own site for a slot that
-// a boundary rule fills).  All eighteen loads are issued together, and a warp
+// source site otherwise.  All eighteen loads are issued together, and a warp
 // issues them once whatever its sites' link masks; the BFL correction of wall
 // links follows as a predicated step.  (4M-site pipe, boundary kernel alone:
 // branching per link 0.0599 ms, pull table for every record 0.0554 ms, run
 // offsets where they apply 0.0541 ms.)
 template <int WALL, bool IO = true>
-__device__ __forceinline__ void gather_general(const StepArgs& a, int g, int s, double* f) {
+__device__ __forceinline__ void gather_links(const StepArgs& a, const Links& l, int s, const int* src, double* f) {
   const GeneralDev& G = a.gen;
-  const uint32_t wm = __ldg(G.wall + g), im = IO ? __ldg(G.iolet + g) : 0u;
-  int src[18];
-  const int run = __ldg(G.run + g);
-  if (run >= 0) {
-    int off[20];
-    load_run_offsets(a, run, off);
-#pragma unroll
-    for (int i = 1; i < Q; i++) src[i - 1] = s + off[i];
-  } else {
-#pragma unroll
-    for (int i = 1; i < Q; i++) src[i - 1] = __ldg(G.src + (int64_t)(i - 1) * G.G + g);
-  }
+  const uint32_t wm = l.wall, im = IO ? l.iolet : 0u;
+  const int g = l.g;
   f[0] = ld(a.fin + s);
 #pragma unroll
   for (int i = 1; i < Q; i++) {
@@ -353,8 +350,16 @@ __device__ __forceinline__ void gather_any(const StepArgs& a, int s, double* f) 
     return;
   }
   const int r = __ldg(a.meta + s);
-  if (r >= 0) gather_bulk(a, s, r, f);
-  else gather_general<WALL>(a, -r - 1, s, f);
+  Links l{0u, 0u, r, 0};
+  if (r < 0) {
+    l.g = -r - 1;
+    l.wall = __ldg(a.gen.wall + l.g);
+    l.iolet = __ldg(a.gen.iolet + l.g);
+    l.run = __ldg(a.gen.run + l.g);
+  }
+  int src[18];
+  load_sources(a, l, s, src);
+  gather_links<WALL>(a, l, s, src, f);
 }
 
 __device__ __forceinline__ void flag_unstable(const StepArgs& a, const double* f) {
@@ -368,12 +373,19 @@ __device__ __forceinline__ void flag_unstable(const StepArgs& a, const double* f
 // Per-site steps
 // ---------------------------------------------------------------------------
 
-// One plain bulk site s of run r.
+// One plain bulk site s (r its run; negative: not a plain bulk site).
 template <int K, bool GATHER, bool MACRO>
 __device__ __forceinline__ void bulk_site_f64(const StepArgs& a, int s, int r) {
   double f[Q];
-  if (GATHER) gather_bulk(a, s, r, f);
-  else {
+  if (GATHER) {
+    int off[20];
+    if (r >= 0) load_run_offsets(a, r, off);
+      if (r < 0) return;
+    f[0] = ld(a.fin + s);
+#pragma unroll
+    for (int i = 1; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + (s + off[i]));
+  } else {
+    if (r < 0) return;
 #pragma unroll
     for (int i = 0; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + s);
   }
@@ -402,18 +414,33 @@ __device__ __forceinline__ void bulk_site_f64(const StepArgs& a, int s, int r) {
   }
 }
 
-// One general (boundary or irregular) site record g.
+// One general (boundary or irregular) site record g.  A GZS wall link's virtual-node value
+// comes from gzs_link_f64, so its slot is not stored here.
 template <int K, int WALL, bool GATHER, bool MACRO, bool IO = true>
 __device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
   const GeneralDev& G = a.gen;
-  const int s = __ldg(G.site + g);
-  const uint32_t wm = __ldg(G.wall + g), im = IO ? __ldg(G.iolet + g) : 0u;
+  Links l{0u, 0u, 0, g};
+  int s = 0;
+  uint32_t keep = ~0u;
   double f[Q];
-  if (GATHER) gather_general<WALL, IO>(a, g, s, f);
-  else {
+  if (GATHER) {
+    int src[18];
+    s = __ldg(G.site + g);
+    l.wall = __ldg(G.wall + g);
+    if (IO) l.iolet = __ldg(G.iolet + g);
+    l.run = __ldg(G.run + g);
+    load_sources(a, l, s, src);
+    if (WALL == kGZS) keep = ~__ldg(G.gzs + g);
+      gather_links<WALL, IO>(a, l, s, src, f);
+  } else {
+    s = __ldg(G.site + g);
+    l.wall = __ldg(G.wall + g);
+    if (IO) l.iolet = __ldg(G.iolet + g);
+    if (WALL == kGZS) keep = ~__ldg(G.gzs + g);
 #pragma unroll
     for (int i = 0; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + s);
   }
+  const uint32_t wm = l.wall, im = l.iolet;
   flag_unstable(a, f);
   double rho, mx, my, mz;
   moments(f, rho, mx, my, mz);
@@ -426,10 +453,6 @@ __device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
   double fp[Q];
 #pragma unroll
   for (int i = 0; i < Q; i++) fp[i] = collide_one<K>(a, f, fneq, om, i);
-  double out[Q];
-#pragma unroll
-  for (int i = 0; i < Q; i++) out[i] = fp[i];
-
   int io = -1;
   if (im) io = __ldg(G.io + g);
   if (im) {
@@ -461,69 +484,10 @@ __device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
       }
     }
   }
-  if (WALL == kGZS && wm) {
-    // GuoZhengShiDelegate::StreamLink (src/lb/streamers/GuoZhengShiDelegate.h:127-293).
+  a.fout[s] = fp[0];
 #pragma unroll
-    for (int d = 1; d < Q; d++) {
-      if (!((wm >> (d - 1)) & 1u)) continue;
-      const int i = inv(d);
-      const double q = (double)__ldg(G.q + (int64_t)(d - 1) * G.G + g);
-      const double fac = 1. - 1. / q;
-      double mw0 = mx * fac, mw1 = my * fac, mw2 = mz * fac;
-      double fnw_i = fneq[i], fnw_d = fneq[d];
-      bool sbb = false;
-      if (q < 0.75) {
-        if ((im >> (i - 1)) & 1u) {
-          const IoletDev& I = a.iolets[io];
-          if (!is_velocity_iolet(I.kind)) {
-            sbb = true;
-          } else {
-            const double p3[3] = {(double)__ldg(G.xyz + g), (double)__ldg(G.xyz + G.G + g), (double)__ldg(G.xyz + 2 * G.G + g)};
-            double nv[3];
-            if (!link_velocity(a, I, io, g, i, false, p3, nv)) {
-              atomicOr(a.status, kStatusIoletRadius);
-              nv[0] = nv[1] = nv[2] = 0.0;
-            }
-            mw0 = q * mw0 + (1. - q) * rho * (nv[0] * (q - 1) / (q + 1));
-            mw1 = q * mw1 + (1. - q) * rho * (nv[1] * (q - 1) / (q + 1));
-            mw2 = q * mw2 + (1. - q) * rho * (nv[2] * (q - 1) / (q + 1));
-          }
-        } else if ((wm >> (i - 1)) & 1u) {
-          sbb = true;
-        } else {
-          const int grun = __ldg(G.run + g);
-          const int nb = grun >= 0 ? s + __ldg(a.run_off + 20 * grun + d) : __ldg(G.src + (int64_t)(d - 1) * G.G + g);
-          double fn[Q];
-          gather_any<WALL, GATHER>(a, nb, fn);
-          double rn, mnx, mny, mnz;
-          moments(fn, rn, mnx, mny, mnz);
-          const double vn0 = mnx / rn, vn1 = mny / rn, vn2 = mnz / rn;
-          const FeqConst fqn(rn, mnx, mny, mnz);
-          mw0 = q * mw0 + (1. - q) * rho * (vn0 * (q - 1) / (q + 1));
-          mw1 = q * mw1 + (1. - q) * rho * (vn1 * (q - 1) / (q + 1));
-          mw2 = q * mw2 + (1. - q) * rho * (vn2 * (q - 1) / (q + 1));
-          fnw_i = q * fnw_i + (1. - q) * (fn[i] - fqn(i));
-          fnw_d = q * fnw_d + (1. - q) * (fn[d] - fqn(d));
-        }
-      }
-      if (sbb) continue;  // slot i reads f*_d, already in out[d]
-      const FeqConst fqw(rho, mw0, mw1, mw2);
-      const double fw_i = fqw(i) + fnw_i;
-      double v;
-      if (K == kTRT) {
-        const int lo = i < d ? i : d;
-        const double fn_lo = lo == i ? fnw_i : fnw_d, fn_hi = lo == i ? fnw_d : fnw_i;
-        const double sym = 0.5 * a.omega * (fn_lo + fn_hi);
-        const double asym = 0.5 * a.omega_minus * (fn_lo - fn_hi);
-        v = i == lo ? (fw_i + sym + asym) : (fw_i + sym - asym);
-      } else {
-        v = fw_i + fnw_i * om;
-      }
-      out[d] = v;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < Q; i++) a.fout[(int64_t)i * a.np + s] = out[i];
+  for (int i = 1; i < Q; i++)
+    if (WALL != kGZS || ((keep >> (i - 1)) & 1u)) a.fout[(int64_t)i * a.np + s] = fp[i];
 
   const int cpl = im ? __ldg(G.cpl + g) : -1;
   if (cpl >= 0) {
@@ -543,6 +507,93 @@ __device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
     }
     if (a.pi) store_pi(a, s, tau, fp, f);
   }
+}
+
+// v[i] for an index known at run time only, without an indexed array.
+__device__ __forceinline__ double pick(const double* v, int i) {
+  double x = v[1];
+#pragma unroll
+  for (int k = 2; k < Q; k++) x = k == i ? v[k] : x;
+  return x;
+}
+
+// Equilibrium of a direction known at run time only.
+__device__ __forceinline__ double feq_at(const FeqConst& c, int i) {
+  const double mde = (double)cx(i) * c.mx + (double)cy(i) * c.my + (double)cz(i) * c.mz;
+  return (i < 7 ? weight(1) : weight(7)) * ((c.t1 + c.nh * (mde * mde)) + 3. * mde);
+}
+
+// The virtual-node value of entry k of the GZS link list (wall link d of general
+// record g; GuoZhengShiDelegate::StreamLink, src/lb/streamers/GuoZhengShiDelegate.h:127-293),
+// stored in f*_d of the record's site.  One thread per link: the site and the
+// neighbour its virtual node extrapolates from are gathered together, where a
+// thread per record walked its links one after the other, each with a gather of its
+// own inlined: 18 gathers of code, most of its time waiting for instructions
+// (594k-site bifurcation, TRT: step 215 -> 105 us).
+template <int K, bool GATHER>
+__device__ __forceinline__ void gzs_link_f64(const StepArgs& a, int k) {
+  const GeneralDev& G = a.gen;
+  const bool live = k < a.gzs_n;
+  const int g = live ? __ldg(a.gzs_rec + k) : 0, d = live ? __ldg(a.gzs_dir + k) : 1;
+  int s = 0, run = 0, i = 0, nb = 0;
+  uint32_t wm = 0, im = 0;
+  double q = 1.0;
+  bool extrapolate = false;
+  if (live) {
+    i = (d & 1) ? d + 1 : d - 1;
+    s = __ldg(G.site + g);
+    wm = __ldg(G.wall + g);
+    im = __ldg(G.iolet + g);
+    run = __ldg(G.run + g);
+    q = (double)__ldg(G.q + (int64_t)(d - 1) * G.G + g);
+    extrapolate = q < 0.75 && !((im >> (i - 1)) & 1u);
+    nb = s;
+    if (extrapolate) nb = run >= 0 ? s + __ldg(a.run_off + 20 * run + d) : __ldg(G.src + (int64_t)(d - 1) * G.G + g);
+  }
+  if (!live) return;
+  double f[Q], fn[Q];
+  gather_any<kGZS, GATHER>(a, s, f);
+  gather_any<kGZS, GATHER>(a, nb, fn);
+  double rho, mx, my, mz;
+  moments(f, rho, mx, my, mz);
+  const FeqConst feq(rho, mx, my, mz);
+  double fnw_i = pick(f, i) - feq_at(feq, i), fnw_d = pick(f, d) - feq_at(feq, d);
+  const double fac = 1. - 1. / q;
+  double mw0 = mx * fac, mw1 = my * fac, mw2 = mz * fac;
+  if (extrapolate) {
+    double rn, mnx, mny, mnz;
+    moments(fn, rn, mnx, mny, mnz);
+    const double vn0 = mnx / rn, vn1 = mny / rn, vn2 = mnz / rn;
+    const FeqConst fqn(rn, mnx, mny, mnz);
+    mw0 = q * mw0 + (1. - q) * rho * (vn0 * (q - 1) / (q + 1));
+    mw1 = q * mw1 + (1. - q) * rho * (vn1 * (q - 1) / (q + 1));
+    mw2 = q * mw2 + (1. - q) * rho * (vn2 * (q - 1) / (q + 1));
+    fnw_i = q * fnw_i + (1. - q) * (pick(fn, i) - feq_at(fqn, i));
+    fnw_d = q * fnw_d + (1. - q) * (pick(fn, d) - feq_at(fqn, d));
+  } else if (q < 0.75) {  // behind the site: a velocity iolet
+    const int io = __ldg(G.io + g);
+    const double p3[3] = {(double)__ldg(G.xyz + g), (double)__ldg(G.xyz + G.G + g), (double)__ldg(G.xyz + 2 * G.G + g)};
+    double nv[3];
+    if (!link_velocity(a, a.iolets[io], io, g, i, false, p3, nv)) {
+      atomicOr(a.status, kStatusIoletRadius);
+      nv[0] = nv[1] = nv[2] = 0.0;
+    }
+    mw0 = q * mw0 + (1. - q) * rho * (nv[0] * (q - 1) / (q + 1));
+    mw1 = q * mw1 + (1. - q) * rho * (nv[1] * (q - 1) / (q + 1));
+    mw2 = q * mw2 + (1. - q) * rho * (nv[2] * (q - 1) / (q + 1));
+  }
+  const FeqConst fqw(rho, mw0, mw1, mw2);
+  const double fw_i = feq_at(fqw, i) + fnw_i;
+  double v;
+  if (K == kTRT) {
+    const double fn_lo = i < d ? fnw_i : fnw_d, fn_hi = i < d ? fnw_d : fnw_i;
+    const double sym = 0.5 * a.omega * (fn_lo + fn_hi);
+    const double asym = 0.5 * a.omega_minus * (fn_lo - fn_hi);
+    v = i < d ? (fw_i + sym + asym) : (fw_i + sym - asym);
+  } else {
+    v = fw_i + fnw_i * a.omega;
+  }
+  a.fout[(int64_t)d * a.np + s] = v;
 }
 
 }  // namespace

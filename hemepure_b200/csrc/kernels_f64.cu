@@ -77,6 +77,12 @@ __global__ void __launch_bounds__(128, (!is_sponge(K) && WALL != kGZS && !MACRO)
   general_site_f64<K, WALL, GATHER, MACRO, false>(a, g);
 }
 
+// The virtual-node values of the GZS wall links, beside the record kernels.
+template <int K, bool GATHER>
+__global__ void __launch_bounds__(128) k_gzs(const StepArgs a) {
+  gzs_link_f64<K, GATHER>(a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 template <int WALL>
 __global__ void __launch_bounds__(256) k_gather(const StepArgs a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -285,6 +291,9 @@ void launch4(const StepArgs& a, int which, int bb, int gb, cudaStream_t st) {
     k_general_walls<K, WALL, GATHER, MACRO><<<(g0 + gb - 1) / gb, gb, 0, st>>>(a);
   if ((which & (kLaunchBoundary | kLaunchIoletRecords)) && a.gen.G > g0)
     k_general<K, WALL, GATHER, MACRO><<<(a.gen.G - g0 + gb - 1) / gb, gb, 0, st>>>(a, g0);
+  if constexpr (WALL == kGZS)
+    if ((which & (kLaunchBoundary | kLaunchWallRecords)) && a.gzs_n > 0)
+      k_gzs<K, GATHER><<<(a.gzs_n + 127) / 128, 128, 0, st>>>(a);
 }
 
 template <int K, int WALL>
@@ -302,7 +311,7 @@ template <int K>
 void launch1(const StepArgs& a, int wall, bool gather, bool macro, int which, int bb, int gb, cudaStream_t st) {
   if (wall == kSBB) launch2<K, kSBB>(a, gather, macro, which, bb, gb, st);
   else if (wall == kBFL) launch2<K, kBFL>(a, gather, macro, which, bb, gb, st);
-  else launch2<K, kGZS>(a, gather, macro, which, bb, gb, st);
+  else if constexpr (K == kLBGK || K == kTRT) launch2<K, kGZS>(a, gather, macro, which, bb, gb, st);  // validate_case
 }
 
 }  // namespace

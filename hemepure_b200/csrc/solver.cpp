@@ -178,6 +178,37 @@ void Solver::upload() {
   upload_vec(g_io_, L_.g_io, tot);
   upload_vec(g_cpl_, L_.g_cpl, tot);
   upload_vec(g_xyz_, L_.g_xyz, tot);
+  // GZS wall links: all but those that bounce back (q < 3/4 with a wall or a
+  // pressure iolet behind the site, src/lb/streamers/GuoZhengShiDelegate.h:127-293).
+  if (opt_.wall == kGZS) {
+    std::vector<uint32_t> mask(L_.G, 0u);
+    for (int g = 0; g < L_.G; g++)
+      for (uint32_t rest = L_.g_wall[g]; rest; rest &= rest - 1) {
+        const int d = __builtin_ctz(rest) + 1, i = inv(d);
+        if (L_.g_q[(size_t)(d - 1) * L_.G + g] < 0.75f) {
+          if ((L_.g_iolet[g] >> (i - 1)) & 1u) {
+            const int idx = L_.g_io[g];
+            if (!is_velocity_iolet((idx < 16 ? p_.inlets[idx] : p_.outlets[idx - 16]).kind)) continue;
+          } else if ((L_.g_wall[g] >> (i - 1)) & 1u) {
+            continue;
+          }
+        }
+        mask[g] |= 1u << (d - 1);
+      }
+    std::vector<int> rec;
+    std::vector<uint8_t> dir;
+    for (int g0 = 0; g0 < L_.G; g0 += 32)
+      for (int d = 1; d < Q; d++)
+        for (int g = g0; g < std::min(L_.G, g0 + 32); g++)
+          if ((mask[g] >> (d - 1)) & 1u) {
+            rec.push_back(g);
+            dir.push_back((uint8_t)d);
+          }
+    gzs_n_ = (int)rec.size();
+    upload_vec(g_gzs_, mask, tot);
+    upload_vec(gzs_rec_, rec, tot);
+    upload_vec(gzs_dir_, dir, tot);
+  }
   // Womersley links: the time-independent factor of the profile at the two points
   // a link's velocity is taken at (the Ladd half-way point, and the neighbour the
   // GZS wall rule extrapolates from), computed once on the host.
@@ -351,6 +382,10 @@ StepArgs Solver::args() const {
   a.gen.cpl = g_cpl_.as<int>();
   a.gen.xyz = g_xyz_.as<int>();
   a.gen.wom = g_wom_.as<int>();
+  a.gen.gzs = g_gzs_.as<uint32_t>();
+  a.gzs_rec = gzs_rec_.as<int>();
+  a.gzs_dir = gzs_dir_.as<uint8_t>();
+  a.gzs_n = gzs_n_;
   a.wom_amp = wom_amp_.as<double>();
   a.tau = p_.tau;
   a.omega = omega_;
