@@ -295,7 +295,7 @@ int hb_pre_send(hb_handle* h) { return h ? HB_OK : HB_ERR_ARG; }
 int hb_pre_receive(hb_handle* h, uint32_t flags) {
   if (!h) return HB_ERR_ARG;
   return guard(h, [&] {
-    h->solver->pre_receive((flags & HB_STEP_MACRO) != 0, 3, (flags & HB_STEP_STRESS) != 0);
+    h->solver->pre_receive((flags & HB_STEP_MACRO) != 0, hb::kLaunchAll, (flags & HB_STEP_STRESS) != 0);
     return HB_OK;
   });
 }

@@ -41,10 +41,12 @@ struct WK3Dev {           // InOutLetWK3 / InOutLetWK2 state
   int pad[2];
 };
 
-// What a step launcher launches (`which`): the plain bulk sites, all boundary
-// records, or the boundary records without iolet links or those with them, for
-// launching the two on separate streams.
-constexpr int kLaunchBulk = 1, kLaunchBoundary = 2, kLaunchWallRecords = 4, kLaunchIoletRecords = 8;
+// What a step launcher launches (`which`) of a steady-state step: the plain bulk
+// sites, the boundary records without iolet links (and the GZS wall links), the
+// boundary records with them.  The first step of a state and the output steps
+// always launch everything.
+constexpr int kLaunchBulk = 1, kLaunchWallRecords = 4, kLaunchIoletRecords = 8;
+constexpr int kLaunchBoundary = kLaunchWallRecords | kLaunchIoletRecords, kLaunchAll = kLaunchBulk | kLaunchBoundary;
 
 struct GeneralDev {
   int G;
@@ -109,9 +111,7 @@ constexpr int kRowA = 32, kRowB = 64, kRowStride = 96;
 enum StatusBits { kStatusUnstable = 1, kStatusIoletRadius = 2, kStatusBadNeighbour = 4 };
 
 // Launchers (kernels_f64.cu).
-// `which`: 1 = plain bulk sites, 2 = general sites, 3 = both.
-void launch_step_f64(const StepArgs& a, int kernel, int wall, bool gather, bool macro, int which, int bulk_block,
-                     int general_block, void* stream);
+void launch_step_f64(const StepArgs& a, int kernel, int wall, bool gather, bool macro, int which, void* stream);
 void launch_gather_f64(const StepArgs& a, int wall, void* stream);
 // Gather the pre-collision f straight into AoS reference order.
 void launch_gather_aos_f64(const StepArgs& a, int wall, const int* st2ref, double* aos, void* stream);

@@ -8,6 +8,7 @@
 
 #include "device.h"
 #include "hb_common.h"
+#include "step_tiles.cuh"
 
 namespace hb {
 namespace {
@@ -255,7 +256,10 @@ __device__ __forceinline__ bool link_velocity(const StepArgs& a, const IoletDev&
   return !(r2a2 > 1.0);
 }
 
-__device__ __forceinline__ double ld(const double* p) { return __ldg(p); }
+// Distributions and ghosts are read with plain loads: the step kernel is launched
+// while the one that wrote them may still be running and waits for it inside
+// (griddepcontrol), which orders plain loads but not the non-coherent ones.
+__device__ __forceinline__ double ld(const double* p) { return *p; }
 
 __device__ __forceinline__ void load_run_offsets(const StepArgs& a, int r, int* off) {
   const int4* o4 = reinterpret_cast<const int4*>(a.run_off) + 5 * r;
@@ -373,22 +377,13 @@ __device__ __forceinline__ void flag_unstable(const StepArgs& a, const double* f
 // Per-site steps
 // ---------------------------------------------------------------------------
 
-// One plain bulk site s (r its run; negative: not a plain bulk site).
+// One plain bulk site s whose run's offsets are `off` (GATHER).
 template <int K, bool GATHER, bool MACRO>
-__device__ __forceinline__ void bulk_site_f64(const StepArgs& a, int s, int r) {
+__device__ __forceinline__ void bulk_site_f64(const StepArgs& a, int s, const int* off) {
   double f[Q];
-  if (GATHER) {
-    int off[20];
-    if (r >= 0) load_run_offsets(a, r, off);
-      if (r < 0) return;
-    f[0] = ld(a.fin + s);
+  f[0] = ld(a.fin + s);
 #pragma unroll
-    for (int i = 1; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + (s + off[i]));
-  } else {
-    if (r < 0) return;
-#pragma unroll
-    for (int i = 0; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + s);
-  }
+  for (int i = 1; i < Q; i++) f[i] = ld(a.fin + (int64_t)i * a.np + (GATHER ? s + off[i] : s));
   flag_unstable(a, f);
   double rho, mx, my, mz;
   moments(f, rho, mx, my, mz);
@@ -414,10 +409,11 @@ __device__ __forceinline__ void bulk_site_f64(const StepArgs& a, int s, int r) {
   }
 }
 
-// One general (boundary or irregular) site record g.  A GZS wall link's virtual-node value
+// One general (boundary or irregular) site record g; `live` false: no record (the
+// thread only waits for the previous step).  A GZS wall link's virtual-node value
 // comes from gzs_link_f64, so its slot is not stored here.
-template <int K, int WALL, bool GATHER, bool MACRO, bool IO = true>
-__device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
+template <int K, int WALL, bool GATHER, bool MACRO, bool IO = true, bool PDL = false>
+__device__ __forceinline__ void general_site_f64(const StepArgs& a, int g, bool live = true) {
   const GeneralDev& G = a.gen;
   Links l{0u, 0u, 0, g};
   int s = 0;
@@ -425,13 +421,17 @@ __device__ __forceinline__ void general_site_f64(const StepArgs& a, int g) {
   double f[Q];
   if (GATHER) {
     int src[18];
-    s = __ldg(G.site + g);
-    l.wall = __ldg(G.wall + g);
-    if (IO) l.iolet = __ldg(G.iolet + g);
-    l.run = __ldg(G.run + g);
-    load_sources(a, l, s, src);
-    if (WALL == kGZS) keep = ~__ldg(G.gzs + g);
-      gather_links<WALL, IO>(a, l, s, src, f);
+    if (live) {
+      s = __ldg(G.site + g);
+      l.wall = __ldg(G.wall + g);
+      if (IO) l.iolet = __ldg(G.iolet + g);
+      l.run = __ldg(G.run + g);
+      load_sources(a, l, s, src);
+      if (WALL == kGZS) keep = ~__ldg(G.gzs + g);
+    }
+    if (PDL) wait_previous_step();
+    if (!live) return;
+    gather_links<WALL, IO>(a, l, s, src, f);
   } else {
     s = __ldg(G.site + g);
     l.wall = __ldg(G.wall + g);
@@ -530,7 +530,7 @@ __device__ __forceinline__ double feq_at(const FeqConst& c, int i) {
 // thread per record walked its links one after the other, each with a gather of its
 // own inlined: 18 gathers of code, most of its time waiting for instructions
 // (594k-site bifurcation, TRT: step 215 -> 105 us).
-template <int K, bool GATHER>
+template <int K, bool GATHER, bool PDL = false>
 __device__ __forceinline__ void gzs_link_f64(const StepArgs& a, int k) {
   const GeneralDev& G = a.gen;
   const bool live = k < a.gzs_n;
@@ -550,6 +550,7 @@ __device__ __forceinline__ void gzs_link_f64(const StepArgs& a, int k) {
     nb = s;
     if (extrapolate) nb = run >= 0 ? s + __ldg(a.run_off + 20 * run + d) : __ldg(G.src + (int64_t)(d - 1) * G.G + g);
   }
+  if (PDL) wait_previous_step();
   if (!live) return;
   double f[Q], fn[Q];
   gather_any<kGZS, GATHER>(a, s, f);

@@ -33,75 +33,20 @@ __device__ __forceinline__ void patch(StepArgs& a, const BatchLatDev& d, int l, 
   a.status = b.lat_status + l;
 }
 
-// Relax the gathered shifted distributions g in place (LBGK, or TRT by pairs of
-// opposite directions, in the arithmetic of collide_one_f), flagging instability
-// in the lattice's status word.  Returns the pre-collision moments.
-__device__ __forceinline__ void relax_inplace(float* g, int* status, bool trt, float om, float omm, float& drho,
-                                              float& mx, float& my, float& mz) {
-  flag_unstable_status(g, status);
-  moments_g(g, drho, mx, my, mz);
-  float eq[Q];
-  GeqF(drho, mx, my, mz).all(eq);  // the same values as GeqF::operator(), by pairs
-  if (trt) {
-    g[0] = g[0] + om * (g[0] - eq[0]);
-#pragma unroll
-    for (int i = 1; i < Q; i += 2) {
-      const int j = i + 1;  // inv(i) for odd i
-      const float fi = g[i] - eq[i], fj = g[j] - eq[j];
-      const float gi = g[i] + 0.5f * om * (fi + fj) + 0.5f * omm * (fi - fj);
-      const float gj = g[j] + 0.5f * om * (fj + fi) + 0.5f * omm * (fj - fi);
-      g[i] = gi;
-      g[j] = gj;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < Q; i++) g[i] = g[i] + (g[i] - eq[i]) * om;
-  }
-}
-
-// Gather of a boundary record with the wall rule chosen at run time (SBB or
-// BFL); the rules are those of gather_general_m.  Every load depends only on
-// the record's metadata and run offsets, and its address is chosen without a
-// branch (records of small vessels side by side in a warp have different link
-// masks), so all are in flight together; the BFL cut distances and own-site
-// values follow in one batch before any arithmetic.
-template <class S>
-__device__ __forceinline__ void gather_general_rt(const StepArgs& a, const MixArgs& m, int gi, int s, uint32_t wm,
-                                                  uint32_t im, int run, const int* off, bool bfl, float* g) {
-  const GeneralDev& G = a.gen;
-  g[0] = ldg_s<S>(m, s);
-#pragma unroll
-  for (int i = 1; i < Q; i++) {
-    const int d = inv(i);
-    const bool bw = (wm >> (d - 1)) & 1u, bi = (im >> (d - 1)) & 1u;
-    const int src = run >= 0 ? s + off[i] : __ldg(G.src + (int64_t)(i - 1) * G.G + gi);
-    const int64_t k = bw ? (int64_t)d * a.np + s : (int64_t)i * a.np + src;
-    g[i] = bi ? __ldg(m.gin + (int64_t)(d - 1) * G.G + gi) : ldg_s<S>(m, k);
-  }
-  if (bfl && wm) {
-    float qv[18], fo[18];
-#pragma unroll
-    for (int i = 1; i < Q; i++) {
-      const int d = inv(i);
-      const bool corr = ((wm >> (d - 1)) & 1u) && !((wm >> (i - 1)) & 1u);
-      qv[i - 1] = corr ? __ldg(G.q + (int64_t)(d - 1) * G.G + gi) : 1.0f;
-      fo[i - 1] = corr ? ldg_s<S>(m, (int64_t)i * a.np + s) : 0.0f;
-    }
-#pragma unroll
-    for (int i = 1; i < Q; i++) {
-      const int d = inv(i);
-      const bool corr = ((wm >> (d - 1)) & 1u) && !((wm >> (i - 1)) & 1u);
-      if (corr) {
-        const float q = qv[i - 1];
-        if (!(q < 0.5f)) g[i] = (g[i] + (2.0f * q - 1.0f) * fo[i - 1]) / (2.0f * q);
-        else g[i] = 2.0f * q * g[i] + (1.0f - 2.0f * q) * g[d];
-      }
-    }
-  }
-}
-
 __device__ __forceinline__ bool lattice_steps(const BatchArgs& b, int l) {
   return b.lat[l].active && !b.lat[l].macro;
+}
+
+// Relax the gathered values in place with the lattice's rates, flagging
+// instability in its status word; returns the pre-collision moments.
+template <class S>
+__device__ __forceinline__ Moments batch_relax(float* g, int* status, const BatchLatDev& d) {
+  const Moments mo(g);
+  if (unstable(g, mo.D, Store<S>::kScale)) atomicOr(status, kStatusUnstable);
+  float neq[Q];
+  non_equilibrium(Geq(mo, Store<S>::kScale), g, neq);
+  relax(g, neq, d.kernel == kTRT, (float)d.omega, (float)d.omega_minus, g);
+  return mo;
 }
 
 // A tile of boundary records, one per thread (walls SBB/BFL, LBGK/TRT).  A
@@ -117,23 +62,26 @@ __device__ __forceinline__ void batch_general_tile(const BatchArgs& b, const Mix
   if (l < 0) return;  // a free boundary slot
   const int s = __ldg(G.site + gi);
   const uint32_t wm = __ldg(G.wall + gi), im = __ldg(G.iolet + gi);
-  const int run = __ldg(G.run + gi);
-  int off[20];
-  if (run >= 0) run_offsets(b.base, run, off);
+  const LinksM links{wm, im, __ldg(G.run + gi), gi};
+  int src[18];
+  load_sources_m(b.base, links, s, src);
   if (!lattice_steps(b, l)) return;
   const BatchLatDev& d = b.lat[l];
   float g[Q];
-  gather_general_rt<S>(b.base, m, gi, s, wm, im, run, off, d.wall == kBFL, g);
-  float drho, mx, my, mz;
-  relax_inplace(g, b.lat_status + l, d.kernel == kTRT, (float)d.omega, (float)d.omega_minus, drho, mx, my, mz);
+  gather_links_m<S>(b.base, m, links, s, src, d.wall == kBFL, g);
+  const Moments mo = batch_relax<S>(g, b.lat_status + l, d);
+  S* o = static_cast<S*>(m.fout) + s;
 #pragma unroll
-  for (int i = 0; i < Q; i++) Store<S>::store(m.fout, (int64_t)i * b.base.np + s, g[i]);
+  for (int i = 0; i < Q; i++) {
+    Store<S>::st(o, g[i]);
+    o += b.base.np;
+  }
   if (im) {
-    const float rho = 1.0f + drho;
-    b.io_moments[gi] = rho;
-    b.io_moments[G.G + gi] = mx / rho;
-    b.io_moments[2 * (int64_t)G.G + gi] = my / rho;
-    b.io_moments[3 * (int64_t)G.G + gi] = mz / rho;
+    const float r = Store<S>::kScale + mo.D;
+    b.io_moments[gi] = 1.0f + mo.D * (1.0f / Store<S>::kScale);
+    b.io_moments[G.G + gi] = mo.mx / r;
+    b.io_moments[2 * (int64_t)G.G + gi] = mo.my / r;
+    b.io_moments[3 * (int64_t)G.G + gi] = mo.mz / r;
   }
 }
 
@@ -155,21 +103,22 @@ __device__ __forceinline__ void batch_bulk_tile(const BatchArgs& b, const MixArg
     if (s[k] >= b.base.n) continue;
     const int r = __ldg(b.base.meta + s[k]);
     if (r < 0) continue;
-    int off[20];
-    run_offsets(b.base, r, off);
-    g[k][0] = ldg_s<S>(m, s[k]);
-#pragma unroll
-    for (int i = 1; i < Q; i++) g[k][i] = ldg_s<S>(m, (int64_t)i * b.base.np + (s[k] + off[i]));
-    if (lattice_steps(b, off[19])) l[k] = off[19];
+    int row[20];
+    load_row(b.base.run_off, r, row);
+    gather_row<S, false>(b.base, m, s[k], row, g[k]);
+    if (lattice_steps(b, row[19])) l[k] = row[19];
   }
 #pragma unroll
   for (int k = 0; k < SPT; k++) {
     if (l[k] < 0) continue;
     const BatchLatDev& d = b.lat[l[k]];
-    float drho, mx, my, mz;
-    relax_inplace(g[k], b.lat_status + l[k], d.kernel == kTRT, (float)d.omega, (float)d.omega_minus, drho, mx, my, mz);
+    batch_relax<S>(g[k], b.lat_status + l[k], d);
+    S* o = static_cast<S*>(m.fout) + s[k];
 #pragma unroll
-    for (int i = 0; i < Q; i++) Store<S>::store(m.fout, (int64_t)i * b.base.np + s[k], g[k][i]);
+    for (int i = 0; i < Q; i++) {
+      Store<S>::st(o, g[k][i]);
+      o += b.base.np;
+    }
   }
 }
 
@@ -178,13 +127,10 @@ __device__ __forceinline__ void batch_bulk_tile(const BatchArgs& b, const MixArg
 // tiles j, j + grid, ..., interleaving the two in proportion, so at any moment
 // the SMs mix latency-bound boundary work with bandwidth-bound bulk work (the
 // assignment is static: no counter, no block-wide barrier).  The kernel is
-// latency-bound, so warps per SM set its speed: with one site per thread it is
-// held to 64 registers (four 256-thread blocks per SM; the boundary path spills
-// ~100 bytes to L1, measured 6-11% faster than 80 registers and three blocks),
-// with two sites per thread to 80 registers (tighter bounds spill the second
-// site's values).
+// latency-bound: with one site per thread it is held to 80 registers (three
+// 256-thread blocks per SM), with two to 128.
 template <class S, int SPT>
-__global__ void __launch_bounds__(256, SPT == 1 ? 4 : 3) k_batch_step(const BatchArgs b) {
+__global__ void __launch_bounds__(256, SPT == 1 ? 3 : 2) k_batch_step(const BatchArgs b) {
   const MixArgs m{b.fin, b.fout, b.gin, b.gout};
   const int j = blockIdx.x, grid = gridDim.x;
   const int n_gen = j < b.gen_tiles ? (b.gen_tiles - j + grid - 1) / grid : 0;
@@ -207,14 +153,12 @@ __global__ void __launch_bounds__(256, SPT == 1 ? 4 : 3) k_batch_step(const Batc
 // The split form of the step: the same tiles as two ordinary (non-persistent)
 // kernels that the graph runs side by side, so each gets its own register
 // budget and the hardware balances the blocks.  Boundary tiles are 128 records;
-// that kernel is latency-bound and held to 48 registers (ten blocks per SM, no
-// spills; 1.6-2% faster on the probe below than at its own 54).  The bulk kernel
-// alone needs 56 registers; held to
-// 40 (six 256-thread blocks per SM, 8 bytes spilled) it ran the serving probe
-// (11 requests, 8.1M sites) at 28.1-28.5k MLUPS against 26.4-27.9k at 56 and
-// 22.9k for the persistent kernel.
+// that kernel is latency-bound.  The bulk kernel runs five blocks of 256 per SM with
+// one site per thread (48 registers, no spills).  Eight lattices, 1.4M sites, FP32,
+// with the shifted forms' arithmetic: 79.4 -> 73.8 us a step (six blocks at 40
+// registers, 68 bytes spilled: 77.0; the persistent kernel 102 -> 82).
 template <class S, int SPT>
-__global__ void __launch_bounds__(256, SPT == 1 ? 6 : 3) k_batch_bulk(const BatchArgs b) {
+__global__ void __launch_bounds__(256, SPT == 1 ? 5 : 3) k_batch_bulk(const BatchArgs b) {
   const MixArgs m{b.fin, b.fout, b.gin, b.gout};
   batch_bulk_tile<S, SPT>(b, m, blockIdx.x);
 }
@@ -260,7 +204,7 @@ __global__ void __launch_bounds__(128) k_batch_ghosts(const BatchArgs b) {
         w[0] = w[1] = w[2] = 0.0f;
       }
       const float corr = 2.0f * wf(link) * rho * (w[0] * cx(link) + w[1] * cy(link) + w[2] * cz(link)) * 3.0f;
-      v = Store<S>::load(b.fout, (int64_t)link * b.base.np + s) - corr;
+      v = Store<S>::ld(static_cast<const S*>(b.fout) + (int64_t)link * b.base.np + s) * (1.0f / Store<S>::kScale) - corr;
     } else {
       const float ux = b.io_moments[G.G + gi], uy = b.io_moments[2 * (int64_t)G.G + gi],
                   uz = b.io_moments[3 * (int64_t)G.G + gi];
@@ -269,8 +213,8 @@ __global__ void __launch_bounds__(128) k_batch_ghosts(const BatchArgs b) {
       const float rbf = (float)rb;
       const float nx = (float)I.nrm_f[0], ny = (float)I.nrm_f[1], nz = (float)I.nrm_f[2];
       const float comp = ux * nx + uy * ny + uz * nz;
-      const GeqF gq(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf);
-      v = gq(inv(link));
+      const Geq gq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f);
+      v = geq_at(gq, inv(link));
     }
     b.gout[(int64_t)(link - 1) * G.G + gi] = v;
   }
@@ -364,7 +308,7 @@ __global__ void k_fill_shift(void* out, int64_t np, int64_t base, int64_t n, Row
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
 #pragma unroll
-  for (int i = 0; i < Q; i++) Store<S>::store(out, (int64_t)i * np + base + s, vals.v[i]);
+  for (int i = 0; i < Q; i++) Store<S>::st(static_cast<S*>(out) + (int64_t)i * np + base + s, vals.v[i] * Store<S>::kScale);
 }
 
 }  // namespace

@@ -24,60 +24,85 @@
 #include "device.h"
 #include "f64_site.cuh"
 #include "hb_common.h"
+#include "step_tiles.cuh"
 
 namespace hb {
 namespace {
 
-constexpr int kGeneralBlocksPerSM = 4;
+constexpr int kStepBlocksPerSM = 4;
 
-// ---------------------------------------------------------------------------
-// Kernels
-// ---------------------------------------------------------------------------
+// One steady-state time step (gathering, no outputs) in one launch: the grid's
+// blocks of kStepBlock threads take boundary records with iolet links, GZS wall
+// links, boundary records without iolet links and plain bulk sites (StepTiles).
+// The bulk blocks are bound by HBM bandwidth and the boundary blocks by latency,
+// so the wall-record blocks are spread evenly among the bulk blocks instead of
+// running ahead of them, and the long iolet and link blocks come first.  The
+// kernel is launched with programmatic dependent launch: its blocks load their
+// constant tables while the previous step drains and wait for it before reading
+// distributions.  Three kernels on three streams, forked and joined by events,
+// before: 13k-site pipe 11.6 -> 7.7 us a step, 497k-site LES stenosis 44.0 -> 34.6,
+// 594k-site GZS bifurcation 105 -> 96, 4M-site pipe 213.5 -> 207.9.  Four blocks of 128 (128 registers, what the BFL gather
+// of the wall records takes) against five (102): 4M-site pipe 214 / 216 us, LES
+// stenosis 36 / 40.
+template <int K, int WALL>
+__global__ void __launch_bounds__(kStepBlock, kStepBlocksPerSM) k_step(const StepArgs a, const StepTiles t) {
+  int b = blockIdx.x;
+  if (b < t.io) {
+    const int g = t.io_first + b * kStepBlock + threadIdx.x;
+    general_site_f64<K, WALL, true, false, true, true>(a, g, g < a.gen.G);
+    return;
+  }
+  b -= t.io;
+  if (WALL == kGZS) {
+    if (b < t.gzs) {
+      gzs_link_f64<K, true, true>(a, b * kStepBlock + threadIdx.x);
+      return;
+    }
+    b -= t.gzs;
+  }
+  const int w = t.walls_before(b);
+  if (t.walls_before(b + 1) > w) {
+    const int g = w * kStepBlock + threadIdx.x;
+    general_site_f64<K, WALL, true, false, false, true>(a, g, g < t.io_first);
+    return;
+  }
+  int s = (b - w) * t.tiles * kStepBlock + threadIdx.x;
+  int r = s < a.n ? __ldg(a.meta + s) : -1;
+  int off[20];
+  if (r >= 0) load_run_offsets(a, r, off);
+  wait_previous_step();
+#pragma unroll 1
+  for (int j = 0; j < t.tiles; j++) {
+    const int s_next = s + kStepBlock;
+    const int r_next = j + 1 < t.tiles && s_next < a.n ? __ldg(a.meta + s_next) : -1;
+    if (r >= 0) bulk_site_f64<K, true, false>(a, s, off);
+    s = s_next;
+    r = r_next;
+    if (r >= 0) load_run_offsets(a, r, off);
+  }
+}
 
-// Three blocks of 256 per SM: TRT otherwise takes 92 registers and runs two
-// (measured 0.228 -> 0.200 ms per launch on the 4M pipe, no spills); LBGK fits
-// in 80 anyway.  The sponge-layer kernels and the output steps would spill under the
-// bound and keep the compiler's allocation.
+// The other forms of the step, as a kernel for the plain bulk sites, one for the
+// boundary records and one for the GZS wall links: the first step of a state
+// (GATHER false: the buffer holds pre-collision values) and the output steps.
 template <int K, bool GATHER, bool MACRO>
-__global__ void __launch_bounds__(256, (is_sponge(K) || MACRO) ? 1 : 3) k_bulk(const StepArgs a) {
+__global__ void __launch_bounds__(256) k_bulk(const StepArgs a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
   const int r = __ldg(a.meta + s);
   if (r < 0) return;
-  bulk_site_f64<K, GATHER, MACRO>(a, s, r);
+  int off[20];
+  if (GATHER) load_run_offsets(a, r, off);
+  bulk_site_f64<K, GATHER, MACRO>(a, s, off);
 }
 
-// The boundary kernel is latency-bound.  Its gather issues the eighteen loads
-// of a record together with the BFL cut distances and own-site values
-// (f64_site.cuh), which needs the registers to hold them: with LBGK or TRT,
-// bounce-back or BFL walls and no outputs it runs four blocks of 128 per SM
-// (125 registers).  4M-site pipe, time alone / whole step: five blocks (96
-// registers, 88 bytes spilled) 0.0523 / 0.2233 ms, four blocks 0.0429 / 0.2171
-// ms; with the BFL loads issued link by link, five blocks 0.0545 / 0.2219 ms and
-// four 0.0585 / 0.2261 ms.  The sponge-layer kernels, GZS walls and output steps
-// keep the compiler's allocation.
 template <int K, int WALL, bool GATHER, bool MACRO>
-__global__ void __launch_bounds__(128, (!is_sponge(K) && WALL != kGZS && !MACRO) ? kGeneralBlocksPerSM : 1)
-    k_general(const StepArgs a, int g0) {
-  const int g = g0 + blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_general(const StepArgs a) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.gen.G) return;
   general_site_f64<K, WALL, GATHER, MACRO>(a, g);
 }
 
-// The records without iolet links (collision types 0 and 1: irregular fluid
-// sites and wall sites, the first bins) in a kernel compiled without the iolet
-// rules, and the rest in k_general after it on the same stream.  4M-site pipe:
-// whole step 0.2165 -> 0.2140 ms (the two launches alone 0.0430 -> 0.0469 ms:
-// the iolet records' short second launch adds its own latency).
-template <int K, int WALL, bool GATHER, bool MACRO>
-__global__ void __launch_bounds__(128, (!is_sponge(K) && WALL != kGZS && !MACRO) ? kGeneralBlocksPerSM : 1)
-    k_general_walls(const StepArgs a) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= a.gen.G_noiolet) return;
-  general_site_f64<K, WALL, GATHER, MACRO, false>(a, g);
-}
-
-// The virtual-node values of the GZS wall links, beside the record kernels.
 template <int K, bool GATHER>
 __global__ void __launch_bounds__(128) k_gzs(const StepArgs a) {
   gzs_link_f64<K, GATHER>(a, blockIdx.x * blockDim.x + threadIdx.x);
@@ -283,35 +308,37 @@ __global__ void k_aos_to_soa(const double* aos, const int* st2ref, int n, double
   soa[(int64_t)i * np + s] = aos[(int64_t)st2ref[s] * Q + i];
 }
 
+template <int K, int WALL>
+void launch_fused(const StepArgs& a, int which, cudaStream_t st) {
+  const StepTiles t = step_tiles(a, which, kStepBlocksPerSM);
+  launch_dependent(k_step<K, WALL>, t.blocks(), st, a, t);
+}
+
+// GZS walls run with LBGK and TRT only (validate_case).
+constexpr bool has_gzs(int k) { return k == kLBGK || k == kTRT; }
+
 template <int K, int WALL, bool GATHER, bool MACRO>
-void launch4(const StepArgs& a, int which, int bb, int gb, cudaStream_t st) {
-  if ((which & 1) && a.n > 0) k_bulk<K, GATHER, MACRO><<<(a.n + bb - 1) / bb, bb, 0, st>>>(a);
-  const int g0 = a.gen.G_noiolet;
-  if ((which & (kLaunchBoundary | kLaunchWallRecords)) && g0 > 0)
-    k_general_walls<K, WALL, GATHER, MACRO><<<(g0 + gb - 1) / gb, gb, 0, st>>>(a);
-  if ((which & (kLaunchBoundary | kLaunchIoletRecords)) && a.gen.G > g0)
-    k_general<K, WALL, GATHER, MACRO><<<(a.gen.G - g0 + gb - 1) / gb, gb, 0, st>>>(a, g0);
-  if constexpr (WALL == kGZS)
-    if ((which & (kLaunchBoundary | kLaunchWallRecords)) && a.gzs_n > 0)
-      k_gzs<K, GATHER><<<(a.gzs_n + 127) / 128, 128, 0, st>>>(a);
+void launch_parts(const StepArgs& a, cudaStream_t st) {
+  if (a.n > 0) k_bulk<K, GATHER, MACRO><<<(a.n + 255) / 256, 256, 0, st>>>(a);
+  if (a.gen.G > 0) k_general<K, WALL, GATHER, MACRO><<<(a.gen.G + 127) / 128, 128, 0, st>>>(a);
+  if constexpr (has_gzs(K))
+    if (a.gzs_n > 0) k_gzs<K, GATHER><<<(a.gzs_n + 127) / 128, 128, 0, st>>>(a);
 }
 
 template <int K, int WALL>
-void launch2(const StepArgs& a, bool gather, bool macro, int which, int bb, int gb, cudaStream_t st) {
-  if (gather) {
-    if (macro) launch4<K, WALL, true, true>(a, which, bb, gb, st);
-    else launch4<K, WALL, true, false>(a, which, bb, gb, st);
-  } else {
-    if (macro) launch4<K, WALL, false, true>(a, which, bb, gb, st);
-    else launch4<K, WALL, false, false>(a, which, bb, gb, st);
-  }
+void launch2(const StepArgs& a, bool gather, bool macro, int which, cudaStream_t st) {
+  if (gather && !macro) launch_fused<K, WALL>(a, which, st);
+  else if (gather) launch_parts<K, WALL, true, true>(a, st);
+  // Without a gather bounce-back and BFL walls have no rule to apply.
+  else if (macro) launch_parts<K, WALL == kBFL ? kSBB : WALL, false, true>(a, st);
+  else launch_parts<K, WALL == kBFL ? kSBB : WALL, false, false>(a, st);
 }
 
 template <int K>
-void launch1(const StepArgs& a, int wall, bool gather, bool macro, int which, int bb, int gb, cudaStream_t st) {
-  if (wall == kSBB) launch2<K, kSBB>(a, gather, macro, which, bb, gb, st);
-  else if (wall == kBFL) launch2<K, kBFL>(a, gather, macro, which, bb, gb, st);
-  else if constexpr (K == kLBGK || K == kTRT) launch2<K, kGZS>(a, gather, macro, which, bb, gb, st);  // validate_case
+void launch1(const StepArgs& a, int wall, bool gather, bool macro, int which, cudaStream_t st) {
+  if (wall == kSBB) launch2<K, kSBB>(a, gather, macro, which, st);
+  else if (wall == kBFL) launch2<K, kBFL>(a, gather, macro, which, st);
+  else if constexpr (has_gzs(K)) launch2<K, kGZS>(a, gather, macro, which, st);
 }
 
 }  // namespace
@@ -371,14 +398,13 @@ void launch_moment_sums(const double* f, int64_t dir_stride, int64_t site_stride
   k_moment_final<<<1, 32, 0, st>>>(scratch, nb, out);
 }
 
-void launch_step_f64(const StepArgs& a, int kernel, int wall, bool gather, bool macro, int which, int bulk_block,
-                     int general_block, void* stream) {
+void launch_step_f64(const StepArgs& a, int kernel, int wall, bool gather, bool macro, int which, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  if (kernel == kLBGK) launch1<kLBGK>(a, wall, gather, macro, which, bulk_block, general_block, st);
-  else if (kernel == kTRT) launch1<kTRT>(a, wall, gather, macro, which, bulk_block, general_block, st);
-  else if (kernel == kLES) launch1<kLES>(a, wall, gather, macro, which, bulk_block, general_block, st);
-  else if (kernel == kLBGKSL) launch1<kLBGKSL>(a, wall, gather, macro, which, bulk_block, general_block, st);
-  else launch1<kTRTSL>(a, wall, gather, macro, which, bulk_block, general_block, st);
+  if (kernel == kLBGK) launch1<kLBGK>(a, wall, gather, macro, which, st);
+  else if (kernel == kTRT) launch1<kTRT>(a, wall, gather, macro, which, st);
+  else if (kernel == kLES) launch1<kLES>(a, wall, gather, macro, which, st);
+  else if (kernel == kLBGKSL) launch1<kLBGKSL>(a, wall, gather, macro, which, st);
+  else launch1<kTRTSL>(a, wall, gather, macro, which, st);
 }
 
 void launch_gather_f64(const StepArgs& a, int wall, void* stream) {

@@ -16,6 +16,64 @@
 namespace hb {
 namespace {
 
+template <class S>
+constexpr int kMixedBlocksPerSM = sizeof(S) == 2 ? 8 : 6;
+
+// One steady-state time step in one launch (k_step of kernels_f64.cu): boundary
+// records with iolet links, GZS wall links, then the other boundary records
+// spread among the plain bulk sites.  Three kernels on three streams before:
+// 197k-site pipe FP32 16.0 -> 10.6 us a step, 187k-site GZS bifurcation 88 -> 23,
+// 1.1M-site LES stenosis 50.7 -> 48.7, 4M-site pipe FP16 92.3 -> 85.1; FP32 stays at
+// 120.0.  The bulk path waits for memory (four fifths of its stalls) rather than
+// issuing: two sites a thread with packed FP32 instructions halve the arithmetic but
+// take 102 registers (FP32 127, FP16 93 us), and the bulk sites in a kernel of their
+// own at 40 registers beside the boundary records measure 121 and 90.
+template <class S, int K, int WALL>
+__global__ void __launch_bounds__(kStepBlock, kMixedBlocksPerSM<S>) k_step_m(const StepArgs a, const MixArgs m, const StepTiles t) {
+  int b = blockIdx.x;
+  if (b < t.io) {
+    const int g = t.io_first + b * kStepBlock + threadIdx.x;
+    general_site_m<S, K, WALL, true, false, true, true>(a, m, g, g < a.gen.G);
+    return;
+  }
+  b -= t.io;
+  if (WALL == kGZS) {
+    if (b < t.gzs) {
+      gzs_link_m<S, K, true, true>(a, m, b * kStepBlock + threadIdx.x);
+      return;
+    }
+    b -= t.gzs;
+  }
+  const int w = t.walls_before(b);
+  if (t.walls_before(b + 1) > w) {
+    const int g = w * kStepBlock + threadIdx.x;
+    general_site_m<S, K, WALL, true, false, false, true>(a, m, g, g < t.io_first);
+    return;
+  }
+  int s = (b - w) * t.tiles * kStepBlock + threadIdx.x;
+  const bool po = a.run_po != nullptr;
+  const int* rows = po ? a.run_po : a.run_off;
+  int r = s < a.n ? __ldg(a.meta + s) : -1;
+  int row[20];
+  if (r >= 0) load_row(rows, r, row);
+  wait_previous_step();
+#pragma unroll 1
+  for (int j = 0; j < t.tiles; j++) {
+    const int s_next = s + kStepBlock;
+    const int r_next = j + 1 < t.tiles && s_next < a.n ? __ldg(a.meta + s_next) : -1;
+    if (r >= 0) {
+      float g[Q];
+      if (po) gather_row<S, true>(a, m, s, row, g);
+      else gather_row<S, false>(a, m, s, row, g);
+      bulk_collide_m<S, K, false>(a, m, s, g);
+    }
+    s = s_next;
+    r = r_next;
+    if (r >= 0) load_row(rows, r, row);
+  }
+}
+// The other forms of the step: the first step of a state (GATHER false) and the
+// output steps.
 template <class S, int K, bool GATHER, bool MACRO>
 __global__ void __launch_bounds__(256) k_bulk_m(const StepArgs a, const MixArgs m) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -25,159 +83,16 @@ __global__ void __launch_bounds__(256) k_bulk_m(const StepArgs a, const MixArgs 
   bulk_site_m<S, K, GATHER, MACRO>(a, m, s, r);
 }
 
-// Two plain bulk sites per thread (s and s + 256 of a 512-site tile), both
-// gathered before either collides: a thread keeps twice the loads in flight,
-// which FP16 storage (2 bytes per load) needs to cover HBM latency.
-template <class S, int K, bool MACRO>
-__global__ void __launch_bounds__(256) k_bulk_m2(const StepArgs a, const MixArgs m) {
-  const int s0 = blockIdx.x * 512 + threadIdx.x, s1 = s0 + 256;
-  const int r0 = s0 < a.n ? __ldg(a.meta + s0) : -1;
-  const int r1 = s1 < a.n ? __ldg(a.meta + s1) : -1;
-  float g0[Q], g1[Q];
-  if (r0 >= 0) gather_bulk_m<S>(a, m, s0, r0, g0);
-  if (r1 >= 0) gather_bulk_m<S>(a, m, s1, r1, g1);
-  if (r0 >= 0) bulk_collide_m<S, K, MACRO>(a, m, s0, g0);
-  if (r1 >= 0) bulk_collide_m<S, K, MACRO>(a, m, s1, g1);
-}
-
-// Steady-state plain bulk sites of the FP16 shifted form (LBGK, TRT; no outputs),
-// SPT sites per thread (s, s + 256, ...), all gathered before any collides (run
-// with one).
-// Each load is one address add: the run table row holds the plane offsets
-// i * np + run_off[i] (Solver::upload).  The collision runs on the stored
-// scale, G = kScale * g (kScale = kHalfScale for FP16, 1 for FP32), so a value
-// is converted but never rescaled on its way in or out: with D = sum G and
-// M = sum c G,
-//   geq_i = w_i (D - 3/2 |M|^2 / (kScale + D) + 9/2 (c_i.M)^2 / (kScale + D) + 3 c_i.M),
-// which is kScale times the unscaled equilibrium of kernels_mixed.cu's header.
-// Opposite directions share the even part of the equilibrium.  The kernel is
-// issue-bound (about 460 instructions a site), so the positivity check compares
-// each value with its constant threshold (one predicated compare; NaN fails it
-// as before) and the stores walk one pointer by the plane stride.  4M-site
-// pipe, FP16 bulk kernel 0.0963 -> 0.0850 ms with the plane offsets, 0.0817 ms
-// with the trimmed check and stores (0.45 -> 0.52 of the measured copy
-// bandwidth), the whole FP16 step 33.1k -> 37.6k MLUPS.  With the instructions
-// trimmed, one site per thread (40 registers, six blocks of 256 per SM) beats
-// two (64 registers, four blocks): 0.0826 -> 0.0779 ms, step 39.3k MLUPS; three
-// sites per thread measured 0.0903 ms, two held to 48 registers 0.0861 ms.
-template <class S>
-struct Lp;
-template <>
-struct Lp<float> {
-  static constexpr float kScale = 1.0f;
-  static __device__ __forceinline__ float ld(const void* base, int64_t k) { return __ldg(static_cast<const float*>(base) + k); }
-  static __device__ __forceinline__ void st(void* base, int64_t k, float v) { static_cast<float*>(base)[k] = v; }
-};
-template <>
-struct Lp<__half> {
-  static constexpr float kScale = kHalfScale;
-  static __device__ __forceinline__ float ld(const void* base, int64_t k) {
-    return __half2float(__ldg(static_cast<const __half*>(base) + k));
-  }
-  static __device__ __forceinline__ void st(void* base, int64_t k, float v) { static_cast<__half*>(base)[k] = __float2half_rn(v); }
-};
-
-template <class S, int K>
-__device__ __forceinline__ void collide_scaled(const StepArgs& a, const MixArgs& m, int s, const float* G) {
-  float D = 0.0f, Mx = 0.0f, My = 0.0f, Mz = 0.0f;
-  bool bad = false;
-#pragma unroll
-  for (int i = 0; i < Q; i++) {
-    D += G[i];
-    Mx += (float)cx(i) * G[i];
-    My += (float)cy(i) * G[i];
-    Mz += (float)cz(i) * G[i];
-    bad |= !(G[i] > -wf(i) * Lp<S>::kScale);
-  }
-  if (bad) atomicOr(a.status, kStatusUnstable);
-  const float inv = 1.0f / (Lp<S>::kScale + D);
-  const float nh = 4.5f * inv;
-  const float t1 = D - 1.5f * (Mx * Mx + My * My + Mz * Mz) * inv;
-  float neq[Q];
-  neq[0] = G[0] - wf(0) * t1;
-#pragma unroll
-  for (int i = 1; i < Q; i += 2) {  // (i, i + 1) are opposite directions
-    const float mde = (float)cx(i) * Mx + (float)cy(i) * My + (float)cz(i) * Mz;
-    const float even = wf(i) * (t1 + nh * mde * mde), odd = wf(i) * (3.0f * mde);
-    neq[i] = G[i] - (even + odd);
-    neq[i + 1] = G[i + 1] - (even - odd);
-  }
-  const float om = (float)a.omega;
-  if (K == kTRT) {
-    const float omm = (float)a.omega_minus;
-    Lp<S>::st(m.fout, s, G[0] + om * neq[0]);
-#pragma unroll
-    for (int i = 1; i < Q; i += 2) {
-      const float sym = 0.5f * om * (neq[i] + neq[i + 1]), asym = 0.5f * omm * (neq[i] - neq[i + 1]);
-      Lp<S>::st(m.fout, (int64_t)i * a.np + s, G[i] + sym + asym);
-      Lp<S>::st(m.fout, (int64_t)(i + 1) * a.np + s, G[i + 1] + sym - asym);
-    }
-  } else {
-    S* o = static_cast<S*>(m.fout) + s;
-#pragma unroll
-    for (int i = 0; i < Q; i++) {
-      Lp<S>::st(o, 0, G[i] + om * neq[i]);
-      o += a.np;
-    }
-  }
-}
-
-template <class S, int K, int SPT>
-__global__ void __launch_bounds__(256) k_bulk_lp(const StepArgs a, const MixArgs m) {
-  const int s0 = blockIdx.x * (256 * SPT) + threadIdx.x;
-  int r[SPT];
-  float G[SPT][Q];
-#pragma unroll
-  for (int k = 0; k < SPT; k++) {
-    const int s = s0 + 256 * k;
-    r[k] = s < a.n ? __ldg(a.meta + s) : -1;
-  }
-#pragma unroll
-  for (int k = 0; k < SPT; k++) {
-    if (r[k] < 0) continue;
-    const int s = s0 + 256 * k;
-    const int4* o4 = reinterpret_cast<const int4*>(a.run_po) + 5 * r[k];
-    int po[20];
-#pragma unroll
-    for (int j = 0; j < 5; j++) {
-      const int4 v = __ldg(o4 + j);
-      po[4 * j] = v.x;
-      po[4 * j + 1] = v.y;
-      po[4 * j + 2] = v.z;
-      po[4 * j + 3] = v.w;
-    }
-#pragma unroll
-    for (int i = 0; i < Q; i++) G[k][i] = Lp<S>::ld(m.fin, (int64_t)s + po[i]);
-  }
-#pragma unroll
-  for (int k = 0; k < SPT; k++)
-    if (r[k] >= 0) collide_scaled<S, K>(a, m, s0 + 256 * k, G[k]);
-}
-
-// The boundary kernel is latency-bound: outside the LES kernel, GZS walls and
-// output steps it runs six blocks of 128 per SM (up to 80 registers), which
-// holds the gather and the BFL loads in flight together (mixed_site.cuh).
-// FP32 on the 4M pipe, time alone / whole step: eight blocks 0.0355 / 0.1231
-// ms, six 0.0326 / 0.1211 ms, five 0.0336 / 0.1227 ms; with the BFL loads
-// issued link by link and eight blocks, 0.0428 / 0.1252 ms.  FP16 storage (its
-// loads half the width) runs eight: 0.0505 / 0.1021 ms at six, 0.0413 / 0.0963
-// ms at eight.
 template <class S, int K, int WALL, bool GATHER, bool MACRO>
-__global__ void __launch_bounds__(128, (K != kLES && WALL != kGZS && !MACRO) ? (sizeof(S) == 2 ? 8 : 6) : 1)
-    k_general_m(const StepArgs a, const MixArgs m, int g0) {
-  const int gi = g0 + blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_general_m(const StepArgs a, const MixArgs m) {
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
   if (gi >= a.gen.G) return;
   general_site_m<S, K, WALL, GATHER, MACRO>(a, m, gi);
 }
 
-// The records without iolet links, compiled without the iolet rules (as the
-// FP64 k_general_walls); k_general_m takes the rest beside it.
-template <class S, int K, int WALL, bool GATHER, bool MACRO>
-__global__ void __launch_bounds__(128, (K != kLES && WALL != kGZS && !MACRO) ? (sizeof(S) == 2 ? 8 : 6) : 1)
-    k_general_m_walls(const StepArgs a, const MixArgs m) {
-  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= a.gen.G_noiolet) return;
-  general_site_m<S, K, WALL, GATHER, MACRO, false>(a, m, gi);
+template <class S, int K, bool GATHER>
+__global__ void __launch_bounds__(128) k_gzs_m(const StepArgs a, const MixArgs m) {
+  gzs_link_m<S, K, GATHER>(a, m, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 template <class S, int WALL, bool GATHER>
@@ -188,7 +103,7 @@ __global__ void __launch_bounds__(256) k_to_aos_m(const StepArgs a, const MixArg
   gather_any_m<S, WALL, GATHER>(a, m, s, g);
   const int64_t base = (int64_t)st2ref[s] * Q;
 #pragma unroll
-  for (int i = 0; i < Q; i++) aos[base + i] = weight(i) + (double)g[i];
+  for (int i = 0; i < Q; i++) aos[base + i] = weight(i) + (double)(g[i] * (1.0f / Store<S>::kScale));
 }
 
 template <class S>
@@ -196,35 +111,33 @@ __global__ void k_from_aos_m(const double* aos, const int* st2ref, int n, int64_
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= (int64_t)n * Q) return;
   const int s = (int)(k / Q), i = (int)(k % Q);
-  Store<S>::store(out, (int64_t)i * np + s, (float)(aos[(int64_t)st2ref[s] * Q + i] - weight(i)));
+  Store<S>::st(static_cast<S*>(out) + (int64_t)i * np + s,
+               (float)(aos[(int64_t)st2ref[s] * Q + i] - weight(i)) * Store<S>::kScale);
 }
 
+// GZS walls run with LBGK and TRT only (validate_case).
+constexpr bool has_gzs(int k) { return k == kLBGK || k == kTRT; }
+
 template <class S, int K, int WALL, bool GATHER, bool MACRO>
-void launch_m4(const StepArgs& a, const MixArgs& m, int which, cudaStream_t st) {
-  if ((which & 1) && a.n > 0) {
-    // FP16 only: FP32 storage measured no faster with it (0.1060 against 0.1060 ms on the
-    // 4M pipe), and keeping FP32 on the general kernel's arithmetic keeps a sharded
-    // FP32 lattice bit-identical to the single lattice.
-    if (GATHER && !MACRO && (K == kLBGK || K == kTRT) && a.run_po && sizeof(S) == 2)
-      k_bulk_lp<S, (K == kTRT ? kTRT : kLBGK), 1><<<(a.n + 255) / 256, 256, 0, st>>>(a, m);
-    else if (GATHER && sizeof(S) == 2) k_bulk_m2<S, K, MACRO><<<(a.n + 511) / 512, 256, 0, st>>>(a, m);
-    else k_bulk_m<S, K, GATHER, MACRO><<<(a.n + 255) / 256, 256, 0, st>>>(a, m);
-  }
-  const int g0 = a.gen.G_noiolet;
-  if ((which & (kLaunchBoundary | kLaunchWallRecords)) && g0 > 0)
-    k_general_m_walls<S, K, WALL, GATHER, MACRO><<<(g0 + 127) / 128, 128, 0, st>>>(a, m);
-  if ((which & (kLaunchBoundary | kLaunchIoletRecords)) && a.gen.G > g0)
-    k_general_m<S, K, WALL, GATHER, MACRO><<<(a.gen.G - g0 + 127) / 128, 128, 0, st>>>(a, m, g0);
+void launch_parts(const StepArgs& a, const MixArgs& m, cudaStream_t st) {
+  if (a.n > 0) k_bulk_m<S, K, GATHER, MACRO><<<(a.n + 255) / 256, 256, 0, st>>>(a, m);
+  if (a.gen.G > 0) k_general_m<S, K, WALL, GATHER, MACRO><<<(a.gen.G + 127) / 128, 128, 0, st>>>(a, m);
+  if constexpr (WALL == kGZS)
+    if (a.gzs_n > 0) k_gzs_m<S, K, GATHER><<<(a.gzs_n + 127) / 128, 128, 0, st>>>(a, m);
 }
 
 template <class S, int K, int WALL>
 void launch_m2(const StepArgs& a, const MixArgs& m, bool gather, bool macro, int which, cudaStream_t st) {
-  if (gather) {
-    if (macro) launch_m4<S, K, WALL, true, true>(a, m, which, st);
-    else launch_m4<S, K, WALL, true, false>(a, m, which, st);
+  if (gather && !macro) {
+    const StepTiles t = step_tiles(a, which, kMixedBlocksPerSM<S>);
+    launch_dependent(k_step_m<S, K, WALL>, t.blocks(), st, a, m, t);
+  } else if (gather) {
+    launch_parts<S, K, WALL, true, true>(a, m, st);
   } else {
-    if (macro) launch_m4<S, K, WALL, false, true>(a, m, which, st);
-    else launch_m4<S, K, WALL, false, false>(a, m, which, st);
+    // Without a gather bounce-back and BFL walls have no rule to apply.
+    constexpr int W = WALL == kBFL ? kSBB : WALL;
+    if (macro) launch_parts<S, K, W, false, true>(a, m, st);
+    else launch_parts<S, K, W, false, false>(a, m, st);
   }
 }
 
@@ -232,7 +145,7 @@ template <class S, int K>
 void launch_m1(const StepArgs& a, const MixArgs& m, int wall, bool gather, bool macro, int which, cudaStream_t st) {
   if (wall == kSBB) launch_m2<S, K, kSBB>(a, m, gather, macro, which, st);
   else if (wall == kBFL) launch_m2<S, K, kBFL>(a, m, gather, macro, which, st);
-  else launch_m2<S, K, kGZS>(a, m, gather, macro, which, st);
+  else if constexpr (has_gzs(K)) launch_m2<S, K, kGZS>(a, m, gather, macro, which, st);
 }
 
 template <class S>

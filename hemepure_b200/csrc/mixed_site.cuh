@@ -1,7 +1,11 @@
 // mixed_site.cuh -- per-site routines of the shifted low-precision forms
 // (g = f - w rho0 stored in FP32 or scaled FP16, FP32 collision), shared by the
-// single-lattice kernels (kernels_mixed.cu) and the batched persistent kernel
+// single-lattice kernels (kernels_mixed.cu) and the batched kernels
 // (kernels_batch.cu).  See kernels_mixed.cu for the formulation.
+//
+// Every routine works on the stored scale, G = kScale * g (kScale = 1 for FP32,
+// kHalfScale for FP16, a power of two, so scaling is exact): a value is converted
+// but never rescaled on its way in or out.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -10,6 +14,7 @@
 #include "../../include/hemeb200.h"
 #include "device.h"
 #include "hb_common.h"
+#include "step_tiles.cuh"
 
 namespace hb {
 namespace {
@@ -17,80 +22,143 @@ namespace {
 template <class S>
 struct Store;
 
+// Plain loads, not the non-coherent path: a step kernel may be launched while the
+// one that wrote its input drains (step_tiles.cuh).
 template <>
 struct Store<float> {
-  static __device__ __forceinline__ float load(const void* p, int64_t k) { return __ldg(static_cast<const float*>(p) + k); }
-  static __device__ __forceinline__ void store(void* p, int64_t k, float v) { static_cast<float*>(p)[k] = v; }
+  static constexpr float kScale = 1.0f;
+  static __device__ __forceinline__ float ld(const float* p) { return *p; }
+  static __device__ __forceinline__ void st(float* p, float v) { *p = v; }
 };
 
-// FP16 holds g * kHalfScale; the scale is a power of two, so scaling is exact.
 template <>
 struct Store<__half> {
-  static __device__ __forceinline__ float load(const void* p, int64_t k) {
-    return __half2float(__ldg(static_cast<const __half*>(p) + k)) * (1.0f / kHalfScale);
-  }
-  static __device__ __forceinline__ void store(void* p, int64_t k, float v) {
-    static_cast<__half*>(p)[k] = __float2half_rn(v * kHalfScale);
-  }
+  static constexpr float kScale = kHalfScale;
+  static __device__ __forceinline__ float ld(const __half* p) { return __half2float(*p); }
+  static __device__ __forceinline__ void st(__half* p, float v) { *p = __float2half_rn(v); }
 };
 
-__device__ __forceinline__ float wf(int i) { return (float)weight(i); }
+__host__ __device__ __forceinline__ constexpr float wf(int i) { return (float)weight(i); }
 
-struct GeqF {
-  float drho, rho, mx, my, mz, t1, nh;
-  __device__ __forceinline__ GeqF(float dr, float x, float y, float z) : drho(dr), mx(x), my(y), mz(z) {
-    rho = 1.0f + drho;
-    const float inv = 1.0f / rho;
-    nh = 4.5f * inv;
-    t1 = drho - 1.5f * (mx * mx + my * my + mz * mz) * inv;
-  }
-  __device__ __forceinline__ float mde(int i) const { return (float)cx(i) * mx + (float)cy(i) * my + (float)cz(i) * mz; }
-  // w_i (t1 + nh (c_i.m)^2) + w_i 3 (c_i.m), each operation rounded as written,
-  // so that all() below gives the same bits.
-  __device__ __forceinline__ float operator()(int i) const {
-    const float e = mde(i);
-    const float even = __fmul_rn(wf(i), __fmaf_rn(__fmul_rn(nh, e), e, t1));
-    const float odd = __fmul_rn(wf(i), __fmul_rn(3.0f, e));
-    return __fadd_rn(even, odd);
-  }
-  // Every direction's value; opposite directions (i, i + 1) share the even part.
-  __device__ __forceinline__ void all(float* out) const {
-    out[0] = (*this)(0);
+// Every operation of the collision is rounded as written here, so a site has the
+// same bits whichever kernel steps it.
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// Density deviation and momentum.  Opposite directions (i, i + 1) enter by their
+// sum and difference.  D - D is 0 for finite values and NaN otherwise: a
+// non-finite value makes every momentum component NaN.
+struct Moments {
+  float D, mx, my, mz;
+  __device__ __forceinline__ explicit Moments(const float* g) {
+    float p[9], m[9];
 #pragma unroll
-    for (int i = 1; i < Q; i += 2) {
-      const float e = mde(i);
-      const float even = __fmul_rn(wf(i), __fmaf_rn(__fmul_rn(nh, e), e, t1));
-      const float odd = __fmul_rn(wf(i), __fmul_rn(3.0f, e));
-      out[i] = __fadd_rn(even, odd);
-      out[i + 1] = __fsub_rn(even, odd);
+    for (int k = 0; k < 9; k++) {
+      p[k] = vadd(g[2 * k + 1], g[2 * k + 2]);
+      m[k] = vsub(g[2 * k + 1], g[2 * k + 2]);
+    }
+    D = vadd(g[0], vadd(vadd(vadd(p[0], p[1]), p[2]),
+                        vadd(vadd(vadd(p[3], p[4]), vadd(p[5], p[6])), vadd(p[7], p[8]))));
+    const float nf = vsub(D, D);
+    mx = vadd(vadd(m[0], nf), vadd(vadd(m[3], m[4]), vadd(m[5], m[6])));
+    my = vadd(vadd(m[1], nf), vadd(vsub(m[3], m[4]), vadd(m[7], m[8])));
+    mz = vadd(vadd(m[2], nf), vadd(vsub(m[5], m[6]), vsub(m[7], m[8])));
+  }
+  __device__ __forceinline__ Moments(float d, float x, float y, float z) : D(d), mx(x), my(y), mz(z) {}
+};
+
+// Shifted equilibrium on the scale `scale`:
+//   w_i (D - 3/2 |M|^2 / (scale + D) + 9/2 (c_i.M)^2 / (scale + D) + 3 c_i.M),
+// with m = 3 M.  The weights enter as they are: the rounded 1/18 and 1/36 add up
+// to a momentum scale of 1 + 7.5e-9, a rounded 3 w of 1/6 to 1 + 3.0e-8, an error
+// that would grow with every step.
+struct Geq {
+  float mx, my, mz, t1, nh;  // 3 M; D - 3/2 |M|^2 / (scale + D); 1/2 / (scale + D)
+  __device__ __forceinline__ Geq(const Moments& m, float scale) {
+    mx = vmul(3.0f, m.mx);
+    my = vmul(3.0f, m.my);
+    mz = vmul(3.0f, m.mz);
+    nh = vmul(0.5f, __frcp_rn(vadd(scale, m.D)));
+    const float mm = vfma(m.mz, mz, vfma(m.my, my, vmul(m.mx, mx)));
+    t1 = vfma(-mm, nh, m.D);
+  }
+  // 3 c_i.M of the odd direction i.
+  __device__ __forceinline__ float mde(int i) const {
+    switch (i) {
+      case 1: return mx;
+      case 3: return my;
+      case 5: return mz;
+      case 7: return vadd(mx, my);
+      case 9: return vsub(mx, my);
+      case 11: return vadd(mx, mz);
+      case 13: return vsub(mx, mz);
+      case 15: return vadd(my, mz);
+      default: return vsub(my, mz);
     }
   }
+  // The odd direction i and its opposite i + 1, which share the even part.
+  __device__ __forceinline__ void pair(int i, float& a, float& b) const {
+    const float w = i < 7 ? wf(1) : wf(7);
+    const float e = mde(i);
+    const float even = vfma(vmul(vmul(w, nh), e), e, vmul(w, t1));
+    a = vfma(w, e, even);
+    b = vfma(-w, e, even);
+  }
+  // Any direction but the rest one.
+  __device__ __forceinline__ float operator()(int i) const {
+    float a, b;
+    pair(i - 1 + (i & 1), a, b);
+    return (i & 1) ? a : b;
+  }
 };
 
-__device__ __forceinline__ void moments_g(const float* g, float& drho, float& mx, float& my, float& mz) {
-  drho = mx = my = mz = 0.0f;
+// G - geq(G).
+__device__ __forceinline__ void non_equilibrium(const Geq& geq, const float* g, float* neq) {
+  neq[0] = vfma(-wf(0), geq.t1, g[0]);
 #pragma unroll
-  for (int i = 0; i < Q; i++) {
-    drho += g[i];
-    mx += (float)cx(i) * g[i];
-    my += (float)cy(i) * g[i];
-    mz += (float)cz(i) * g[i];
+  for (int i = 1; i < Q; i += 2) {
+    float a, b;
+    geq.pair(i, a, b);
+    neq[i] = vsub(g[i], a);
+    neq[i + 1] = vsub(g[i + 1], b);
   }
 }
 
-__device__ __forceinline__ float les_tau_f(const StepArgs& a, const float* fneq, float vt) {
-  const float tau0 = (float)a.tau;
-  float q12 = 0.0f;
+// Post-collision values: G + om neq, or TRT with the rates of the even and odd parts.
+__device__ __forceinline__ void relax(const float* g, const float* neq, bool trt, float om, float omm, float* out) {
+  out[0] = vfma(om, neq[0], g[0]);
+  if (trt) {
+    const float hp = vmul(0.5f, om), hm = vmul(0.5f, omm), hn = vmul(-0.5f, omm);
 #pragma unroll
-  for (int p = 0; p < 3; p++)
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      float qij = 0.0f;
-#pragma unroll
-      for (int v = 0; v < Q; v++) qij += (float)(cc(p, v) * cc(r, v)) * fneq[v];
-      q12 += qij * qij;
+    for (int i = 1; i < Q; i += 2) {
+      const float s = vadd(neq[i], neq[i + 1]), d = vsub(neq[i], neq[i + 1]);
+      out[i] = vfma(hm, d, vfma(hp, s, g[i]));
+      out[i + 1] = vfma(hn, d, vfma(hp, s, g[i + 1]));
     }
-  q12 = sqrtf(q12);
+  } else {
+#pragma unroll
+    for (int i = 1; i < Q; i++) out[i] = vfma(om, neq[i], g[i]);
+  }
+}
+
+// Some f <= 0 (or NaN): the smallest value of each weight against -w, with D for
+// the NaN that a minimum drops.
+__device__ __forceinline__ bool unstable(const float* g, float D, float scale) {
+  float a = fminf(fminf(g[1], g[2]), g[3]), d = fminf(fminf(g[7], g[8]), g[9]);
+  a = fminf(fminf(a, g[4]), fminf(g[5], g[6]));
+  d = fminf(fminf(d, g[10]), g[11]);
+  d = fminf(fminf(d, g[12]), g[13]);
+  d = fminf(fminf(d, g[14]), g[15]);
+  d = fminf(fminf(d, g[16]), fminf(g[17], g[18]));
+  return !(g[0] > -wf(0) * scale) || !(a > -wf(1) * scale) || !(d > -wf(7) * scale) || D != D;
+}
+
+// Relaxation time of the LES kernel from the squared non-equilibrium flux.
+__device__ __forceinline__ float les_tau_of(const StepArgs& a, float q12sq, float vt) {
+  const float tau0 = (float)a.tau;
+  const float q12 = sqrtf(q12sq);
   const float ks = (float)(18.0 * 1.4142135623730950488016887242097 * 0.01);
   const float tau_les = 0.5f * (tau0 + sqrtf(tau0 * tau0 + ks * q12));
   if (a.t <= a.lifetime / 2) return (vt == tau0) ? tau_les : vt;
@@ -98,63 +166,62 @@ __device__ __forceinline__ float les_tau_f(const StepArgs& a, const float* fneq,
   return tau_les;
 }
 
-template <int K>
-__device__ __forceinline__ float collide_one_f(const StepArgs& a, const float* g, const float* fneq, float om, int i) {
-  if (K == kTRT) {
-    const float op = (float)a.omega, omm = (float)a.omega_minus;
-    if (i == 0) return g[0] + op * fneq[0];
-    const int j = inv(i);
-    const float sym = 0.5f * op * (fneq[i] + fneq[j]);
-    const float asym = 0.5f * omm * (fneq[i] - fneq[j]);
-    return g[i] + sym + asym;
-  }
-  return g[i] + fneq[i] * om;
+// Sum of v[l] c_p c_r: the fluxes of opposite directions enter by their sum.
+__device__ __forceinline__ void fluxes(const float* v, float& xx, float& xy, float& xz, float& yy, float& yz, float& zz) {
+  float s[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) s[k] = vadd(v[2 * k + 1], v[2 * k + 2]);
+  const float a = vadd(s[3], s[4]), b = vadd(s[5], s[6]), c = vadd(s[7], s[8]);
+  xx = vadd(s[0], vadd(a, b));
+  yy = vadd(s[1], vadd(a, c));
+  zz = vadd(s[2], vadd(b, c));
+  xy = vsub(s[3], s[4]);
+  xz = vsub(s[5], s[6]);
+  yz = vsub(s[7], s[8]);
 }
 
-__device__ __forceinline__ double wss_mag_f(float tau, const float* gp, const float* g, const float nor[3]) {
-  float pi[3][3];
-#pragma unroll
-  for (int p = 0; p < 3; p++)
-#pragma unroll
-    for (int r = 0; r <= p; r++) {
-      float acc = 0.0f;
-#pragma unroll
-      for (int l = 0; l < Q; l++) acc += (gp[l] - g[l]) * (float)(cc(p, l) * cc(r, l));
-      pi[p][r] = acc * -(tau - 0.5f);
-    }
-  pi[0][1] = pi[1][0];
-  pi[0][2] = pi[2][0];
-  pi[1][2] = pi[2][1];
-  float sq = 0.0f, ns = 0.0f;
-#pragma unroll
-  for (int p = 0; p < 3; p++) {
-    const float sv = pi[p][0] * nor[0] + pi[p][1] * nor[1] + pi[p][2] * nor[2];
-    sq += sv * sv;
-    ns += sv * nor[p];
+__device__ __forceinline__ float flux_norm_sq(const float* neq) {
+  float xx, xy, xz, yy, yz, zz;
+  fluxes(neq, xx, xy, xz, yy, yz, zz);
+  const float off = vfma(yz, yz, vfma(xz, xz, vmul(xy, xy)));
+  return vfma(2.0f, off, vfma(zz, zz, vfma(yy, yy, vmul(xx, xx))));
+}
+
+// The site's relaxation time and rate for kernel K (LES: from its non-equilibrium part).
+template <class S, int K>
+__device__ __forceinline__ void site_rate(const StepArgs& a, const float* neq, int s, float& tau, float& om) {
+  om = (float)a.omega;
+  tau = (float)a.tau;
+  if (K == kLES) {
+    tau = les_tau_of(a, flux_norm_sq(neq) * (1.0f / (Store<S>::kScale * Store<S>::kScale)), (float)__ldg(a.vtau + s));
+    om = -1.0f / tau;
   }
+}
+
+// Momentum flux tensor of an output step (unscaled), -(tau - 1/2) sum (gp - g) c c.
+template <class S>
+__device__ __forceinline__ void flux_tensor(float tau, const float* gp, const float* g, float pi[6]) {
+  float df[Q];
+#pragma unroll
+  for (int l = 0; l < Q; l++) df[l] = gp[l] - g[l];
+  fluxes(df, pi[0], pi[1], pi[2], pi[3], pi[4], pi[5]);
+#pragma unroll
+  for (int k = 0; k < 6; k++) pi[k] = pi[k] * (1.0f / Store<S>::kScale) * -(tau - 0.5f);
+}
+
+__device__ __forceinline__ double wss_mag_f(const float pi[6], const float nor[3]) {
+  const float sx = pi[0] * nor[0] + pi[1] * nor[1] + pi[2] * nor[2];
+  const float sy = pi[1] * nor[0] + pi[3] * nor[1] + pi[4] * nor[2];
+  const float sz = pi[2] * nor[0] + pi[4] * nor[1] + pi[5] * nor[2];
+  const float sq = sx * sx + sy * sy + sz * sz, ns = sx * nor[0] + sy * nor[1] + sz * nor[2];
   return (double)sqrtf(fmaxf(sq - ns * ns, 0.0f));
 }
 
-// Momentum flux tensor of an output step for the stress caches (FP32 sums of the
-// shifted values: gp - g equals fp - f), stored as FP64 like store_pi.
-__device__ __forceinline__ void store_pi_f(const StepArgs& a, int s, float tau, const float* gp, const float* g) {
-  float pi[3][3];
-#pragma unroll
-  for (int p = 0; p < 3; p++)
-#pragma unroll
-    for (int r = 0; r <= p; r++) {
-      float acc = 0.0f;
-#pragma unroll
-      for (int l = 0; l < Q; l++) acc += (gp[l] - g[l]) * (float)(cc(p, l) * cc(r, l));
-      pi[p][r] = acc * -(tau - 0.5f);
-    }
+// The tensor as the stress caches read it (FP64, like store_pi), then tau.
+__device__ __forceinline__ void store_pi_f(const StepArgs& a, int s, float tau, const float pi[6]) {
   double* o = a.pi + s;
-  o[0] = (double)pi[0][0];
-  o[a.np] = (double)pi[1][0];
-  o[2 * a.np] = (double)pi[2][0];
-  o[3 * a.np] = (double)pi[1][1];
-  o[4 * a.np] = (double)pi[2][1];
-  o[5 * a.np] = (double)pi[2][2];
+#pragma unroll
+  for (int k = 0; k < 6; k++) o[k * a.np] = (double)pi[k];
   o[6 * a.np] = (double)tau;
 }
 
@@ -198,20 +265,23 @@ __device__ __forceinline__ bool link_velocity_f(const StepArgs& a, const IoletDe
   return !(r2a2 > 1.0);
 }
 
-__device__ __forceinline__ void run_offsets(const StepArgs& a, int r, int* off) {
-  const int4* o4 = reinterpret_cast<const int4*>(a.run_off) + 5 * r;
+// One 20-entry row of the run table (run offsets or plane offsets).
+__device__ __forceinline__ void load_row(const int* table, int r, int* row) {
+  const int4* o4 = reinterpret_cast<const int4*>(table) + 5 * (int64_t)r;
 #pragma unroll
   for (int k = 0; k < 5; k++) {
     const int4 v = __ldg(o4 + k);
-    off[4 * k] = v.x;
-    off[4 * k + 1] = v.y;
-    off[4 * k + 2] = v.z;
-    off[4 * k + 3] = v.w;
+    row[4 * k] = v.x;
+    row[4 * k + 1] = v.y;
+    row[4 * k + 2] = v.z;
+    row[4 * k + 3] = v.w;
   }
 }
 
 // Arguments of the shifted kernels: StepArgs for the shared tables, plus typed
-// storage pointers (fin/fout/gin/gout of StepArgs are unused here).
+// storage pointers (fin/fout/gin/gout of StepArgs are unused here).  Ghost values
+// are FP32 and unscaled; StepArgs' cut distances hold the BFL coefficient (below)
+// except for GZS walls.
 struct MixArgs {
   const void* fin;
   void* fout;
@@ -219,86 +289,78 @@ struct MixArgs {
   float* gout;
 };
 
-template <class S>
-__device__ __forceinline__ float ldg_s(const MixArgs& m, int64_t k) { return Store<S>::load(m.fin, k); }
-
-template <class S>
-__device__ __forceinline__ void gather_bulk_m(const StepArgs& a, const MixArgs& m, int s, int r, float* g) {
-  if (a.run_po) {
-    // The run table's plane offsets i * np + run_off[i]: one add per load.
-    const int4* o4 = reinterpret_cast<const int4*>(a.run_po) + 5 * r;
-    int po[20];
+// Gather of a plain bulk site from its run row: plane offsets i * np + run_off[i]
+// (PO: one address add per load) or run offsets.
+template <class S, bool PO>
+__device__ __forceinline__ void gather_row(const StepArgs& a, const MixArgs& m, int s, const int* row, float* g) {
+  const S* p = static_cast<const S*>(m.fin) + s;
+  g[0] = Store<S>::ld(p);
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-      const int4 v = __ldg(o4 + k);
-      po[4 * k] = v.x;
-      po[4 * k + 1] = v.y;
-      po[4 * k + 2] = v.z;
-      po[4 * k + 3] = v.w;
-    }
-    const S* base = static_cast<const S*>(m.fin) + s;
-#pragma unroll
-    for (int i = 0; i < Q; i++) g[i] = Store<S>::load(base, po[i]);
-    return;
+  for (int i = 1; i < Q; i++) {
+    if (!PO) p += a.np;
+    g[i] = Store<S>::ld(p + row[i]);
   }
-  int off[20];
-  run_offsets(a, r, off);
-  g[0] = ldg_s<S>(m, s);
+}
+
+// Link masks and run of a site: a general record's own, none for a plain bulk site.
+struct LinksM {
+  uint32_t wall, iolet;
+  int run, g;
+};
+
+__device__ __forceinline__ void load_sources_m(const StepArgs& a, const LinksM& l, int s, int* src) {
+  if (l.run >= 0) {
+    int off[20];
+    load_row(a.run_off, l.run, off);
 #pragma unroll
-  for (int i = 1; i < Q; i++) g[i] = ldg_s<S>(m, (int64_t)i * a.np + (s + off[i]));
+    for (int i = 1; i < Q; i++) src[i - 1] = s + off[i];
+  } else {
+#pragma unroll
+    for (int i = 1; i < Q; i++) src[i - 1] = __ldg(a.gen.src + (int64_t)(i - 1) * a.gen.G + l.g);
+  }
 }
 
 // Every slot's first value is one load (predicated between the ghost buffer and
 // the distributions, with no branch on the link masks): the ghost of an iolet
 // link, g*_d of the own site for a wall link, g*_i of the source site otherwise
 // (s + run offset for a record that follows its run, else its pull table).  The
-// BFL correction of wall links follows as a predicated step (as the FP64 kernel).
-template <class S, int WALL, bool IO = true>
-__device__ __forceinline__ void gather_general_m(const StepArgs& a, const MixArgs& m, int gi, int s, float* g) {
+// BFL correction of wall links follows as a predicated step: both of its rules
+// (gather_links, f64_site.cuh) are g*_d + |c| (X - g*_d) with the coefficient c of
+// bfl_coefficient laid out once per link, so the kernels divide by nothing here.
+template <class S, bool IO = true>
+__device__ __forceinline__ void gather_links_m(const StepArgs& a, const MixArgs& m, const LinksM& l, int s, const int* src,
+                                               bool bfl, float* g) {
   const GeneralDev& G = a.gen;
-  const uint32_t wm = __ldg(G.wall + gi), im = IO ? __ldg(G.iolet + gi) : 0u;
-  const int run = __ldg(G.run + gi);
-  int src[18];
-  if (run >= 0) {
-    int off[20];
-    run_offsets(a, run, off);
-#pragma unroll
-    for (int i = 1; i < Q; i++) src[i - 1] = s + off[i];
-  } else {
-#pragma unroll
-    for (int i = 1; i < Q; i++) src[i - 1] = __ldg(G.src + (int64_t)(i - 1) * G.G + gi);
-  }
-  g[0] = ldg_s<S>(m, s);
+  const uint32_t wm = l.wall, im = IO ? l.iolet : 0u;
+  const S* fin = static_cast<const S*>(m.fin);
+  g[0] = Store<S>::ld(fin + s);
 #pragma unroll
   for (int i = 1; i < Q; i++) {
     const int d = inv(i);
     const bool bw = (wm >> (d - 1)) & 1u, bi = (im >> (d - 1)) & 1u;
     const int64_t k = bw ? (int64_t)d * a.np + s : (int64_t)i * a.np + src[i - 1];
     float v;
-    if (bi) v = __ldg(m.gin + (int64_t)(d - 1) * G.G + gi);
-    else v = ldg_s<S>(m, k);
+    if (bi) v = m.gin[(int64_t)(d - 1) * G.G + l.g] * Store<S>::kScale;
+    else v = Store<S>::ld(fin + k);
     g[i] = v;
   }
-  if (WALL == kBFL && wm) {
-    // The BFL rule of gather_general (f64_site.cuh), in FP32 on the stored
-    // deviations; cut distances and own-site values loaded before any arithmetic.
-    float qv[18], fo[18];
+  if (bfl && wm) {
+    float cv[18], fo[18];
 #pragma unroll
     for (int i = 1; i < Q; i++) {
       const int d = inv(i);
       const bool corr = ((wm >> (d - 1)) & 1u) && !((wm >> (i - 1)) & 1u);
-      qv[i - 1] = corr ? __ldg(G.q + (int64_t)(d - 1) * G.G + gi) : 1.0f;
-      fo[i - 1] = corr ? ldg_s<S>(m, (int64_t)i * a.np + s) : 0.0f;
+      cv[i - 1] = corr ? __ldg(G.q + (int64_t)(d - 1) * G.G + l.g) : 0.0f;
+      fo[i - 1] = corr ? Store<S>::ld(fin + (int64_t)i * a.np + s) : 0.0f;
     }
+    // Slot d of a corrected link is a plain gather (no wall behind the site): the
+    // pre-correction values below are final ones.
 #pragma unroll
     for (int i = 1; i < Q; i++) {
       const int d = inv(i);
-      const bool corr = ((wm >> (d - 1)) & 1u) && !((wm >> (i - 1)) & 1u);
-      if (corr) {
-        const float q = qv[i - 1];
-        if (!(q < 0.5f)) g[i] = (g[i] + (2.0f * q - 1.0f) * fo[i - 1]) / (2.0f * q);
-        else g[i] = 2.0f * q * g[i] + (1.0f - 2.0f * q) * g[d];
-      }
+      const float c = cv[i - 1];
+      const float x = c > 0.0f ? fo[i - 1] : g[d];
+      if (c != 0.0f) g[i] = vfma(fabsf(c), vsub(x, g[i]), g[i]);
     }
   }
 }
@@ -306,114 +368,131 @@ __device__ __forceinline__ void gather_general_m(const StepArgs& a, const MixArg
 template <class S, int WALL, bool GATHER>
 __device__ __forceinline__ void gather_any_m(const StepArgs& a, const MixArgs& m, int s, float* g) {
   if (!GATHER) {
+    const S* p = static_cast<const S*>(m.fin) + s;
 #pragma unroll
-    for (int i = 0; i < Q; i++) g[i] = ldg_s<S>(m, (int64_t)i * a.np + s);
+    for (int i = 0; i < Q; i++) g[i] = Store<S>::ld(p + (int64_t)i * a.np);
     return;
   }
   const int r = __ldg(a.meta + s);
-  if (r >= 0) gather_bulk_m<S>(a, m, s, r, g);
-  else gather_general_m<S, WALL>(a, m, -r - 1, s, g);
+  LinksM l{0u, 0u, r, 0};
+  if (r < 0) {
+    l.g = -r - 1;
+    l.wall = __ldg(a.gen.wall + l.g);
+    l.iolet = __ldg(a.gen.iolet + l.g);
+    l.run = __ldg(a.gen.run + l.g);
+  }
+  int src[18];
+  load_sources_m(a, l, s, src);
+  gather_links_m<S>(a, m, l, s, src, WALL == kBFL, g);
 }
 
-__device__ __forceinline__ void flag_unstable_status(const float* g, int* status) {
-  bool bad = false;
-#pragma unroll
-  for (int i = 0; i < Q; i++) bad |= !(g[i] > -wf(i));
-  if (bad) atomicOr(status, kStatusUnstable);
+// Macroscopic outputs of a site from its moments (and, at a wall site, its stress).
+template <class S>
+__device__ __forceinline__ void store_macro(const StepArgs& a, int s, const Moments& mo, float tau, const float* gp,
+                                            const float* g, bool wall, const float nor[3]) {
+  const float r = Store<S>::kScale + mo.D;
+  a.rho[s] = (double)(1.0f + mo.D * (1.0f / Store<S>::kScale));
+  a.u[s] = (double)(mo.mx / r);
+  a.u[a.np + s] = (double)(mo.my / r);
+  a.u[2 * a.np + s] = (double)(mo.mz / r);
+  if (!wall && !a.pi) {
+    a.wss[s] = kNoValue;
+    return;
+  }
+  float pi[6];
+  flux_tensor<S>(tau, gp, g, pi);
+  a.wss[s] = wall ? wss_mag_f(pi, nor) : kNoValue;
+  if (a.pi) store_pi_f(a, s, tau, pi);
 }
 
-__device__ __forceinline__ void flag_unstable_m(const StepArgs& a, const float* g) { flag_unstable_status(g, a.status); }
-
-// Collision and store of plain bulk site s from its pre-collision g.  The bulk
-// kernels issue about 490 instructions a site for 152 bytes (FP32), so the
-// equilibrium is evaluated by pairs of opposite directions and the stores walk
-// one pointer (4M pipe, FP32 bulk kernel 0.1065 -> 0.1038 ms, 0.83 -> 0.85 of
-// the measured copy bandwidth).
+// One plain bulk site s from its gathered values.
 template <class S, int K, bool MACRO>
 __device__ __forceinline__ void bulk_collide_m(const StepArgs& a, const MixArgs& m, int s, const float* g) {
-  flag_unstable_m(a, g);
-  float drho, mx, my, mz;
-  moments_g(g, drho, mx, my, mz);
-  const GeqF geq(drho, mx, my, mz);
-  float fneq[Q];
-  geq.all(fneq);
+  float neq[Q], gp[Q];
+  const Moments mo(g);
+  if (unstable(g, mo.D, Store<S>::kScale)) atomicOr(a.status, kStatusUnstable);
+  non_equilibrium(Geq(mo, Store<S>::kScale), g, neq);
+  float tau, om;
+  site_rate<S, K>(a, neq, s, tau, om);
+  relax(g, neq, K == kTRT, om, (float)a.omega_minus, gp);
+  S* o = static_cast<S*>(m.fout) + s;
 #pragma unroll
-  for (int i = 0; i < Q; i++) fneq[i] = g[i] - fneq[i];
-  float om = (float)a.omega, tau = (float)a.tau;
-  if (K == kLES) {
-    tau = les_tau_f(a, fneq, (float)__ldg(a.vtau + s));
-    om = -1.0f / tau;
-  }
-  {
-    S* o = static_cast<S*>(m.fout) + s;
-#pragma unroll
-    for (int i = 0; i < Q; i++) {
-      Store<S>::store(o, 0, collide_one_f<K>(a, g, fneq, om, i));
-      o += a.np;
-    }
+  for (int i = 0; i < Q; i++) {
+    Store<S>::st(o, gp[i]);
+    o += a.np;
   }
   if (MACRO) {
-    const float rho = 1.0f + drho;
-    a.rho[s] = (double)rho;
-    a.u[s] = (double)(mx / rho);
-    a.u[a.np + s] = (double)(my / rho);
-    a.u[2 * a.np + s] = (double)(mz / rho);
-    a.wss[s] = kNoValue;
-    if (a.pi) {
-      float gp[Q];
-#pragma unroll
-      for (int i = 0; i < Q; i++) gp[i] = collide_one_f<K>(a, g, fneq, om, i);
-      store_pi_f(a, s, tau, gp, g);
-    }
+    const float nor[3] = {0.0f, 0.0f, 0.0f};
+    store_macro<S>(a, s, mo, tau, gp, g, false, nor);
   }
 }
 
-// One plain bulk site s of run r (k_bulk_m, and the batched kernel).
+// One plain bulk site s (the output steps and the first step of a state).
 template <class S, int K, bool GATHER, bool MACRO>
 __device__ __forceinline__ void bulk_site_m(const StepArgs& a, const MixArgs& m, int s, int r) {
   float g[Q];
-  if (GATHER) gather_bulk_m<S>(a, m, s, r, g);
-  else {
+  if (GATHER) {
+    int off[20];
+    load_row(a.run_off, r, off);
+    gather_row<S, false>(a, m, s, off, g);
+  } else {
+    const S* p = static_cast<const S*>(m.fin) + s;
 #pragma unroll
-    for (int i = 0; i < Q; i++) g[i] = ldg_s<S>(m, (int64_t)i * a.np + s);
+    for (int i = 0; i < Q; i++) g[i] = Store<S>::ld(p + (int64_t)i * a.np);
   }
   bulk_collide_m<S, K, MACRO>(a, m, s, g);
 }
 
-// One general site gi (k_general_m, and the batched kernel).
-template <class S, int K, int WALL, bool GATHER, bool MACRO, bool IO = true>
-__device__ __forceinline__ void general_site_m(const StepArgs& a, const MixArgs& m, int gi) {
+// One general site gi (`live` false: no record; the thread only waits for the
+// previous step).  A GZS wall link's virtual-node value comes from gzs_link_m, so
+// its slot is not stored here.
+template <class S, int K, int WALL, bool GATHER, bool MACRO, bool IO = true, bool PDL = false>
+__device__ __forceinline__ void general_site_m(const StepArgs& a, const MixArgs& m, int gi, bool live = true) {
   const GeneralDev& G = a.gen;
-  const int s = __ldg(G.site + gi);
-  const uint32_t wm = __ldg(G.wall + gi), im = IO ? __ldg(G.iolet + gi) : 0u;
+  constexpr float kScale = Store<S>::kScale;
+  LinksM l{0u, 0u, 0, gi};
+  int s = 0;
+  uint32_t keep = ~0u;
   float g[Q];
-  if (GATHER) gather_general_m<S, WALL, IO>(a, m, gi, s, g);
-  else {
-#pragma unroll
-    for (int i = 0; i < Q; i++) g[i] = ldg_s<S>(m, (int64_t)i * a.np + s);
+  if (live) {
+    s = __ldg(G.site + gi);
+    l.wall = __ldg(G.wall + gi);
+    if (IO) l.iolet = __ldg(G.iolet + gi);
+    if (WALL == kGZS) keep = ~__ldg(G.gzs + gi);
   }
-  flag_unstable_m(a, g);
-  float drho, mx, my, mz;
-  moments_g(g, drho, mx, my, mz);
-  const float rho = 1.0f + drho;
-  const float ux = mx / rho, uy = my / rho, uz = mz / rho;
-  const GeqF geq(drho, mx, my, mz);
-  float fneq[Q];
+  if (GATHER) {
+    int src[18];
+    if (live) {
+      l.run = __ldg(G.run + gi);
+      load_sources_m(a, l, s, src);
+    }
+    if (PDL) wait_previous_step();
+    if (!live) return;
+    gather_links_m<S, IO>(a, m, l, s, src, WALL == kBFL, g);
+  } else {
+    const S* p = static_cast<const S*>(m.fin) + s;
 #pragma unroll
-  for (int i = 0; i < Q; i++) fneq[i] = g[i] - geq(i);
-  float om = (float)a.omega, tau = (float)a.tau;
-  if (K == kLES) {
-    tau = les_tau_f(a, fneq, (float)__ldg(a.vtau + s));
-    om = -1.0f / tau;
+    for (int i = 0; i < Q; i++) g[i] = Store<S>::ld(p + (int64_t)i * a.np);
   }
-  float gp[Q], out[Q];
+  const Moments mo(g);
+  if (unstable(g, mo.D, kScale)) atomicOr(a.status, kStatusUnstable);
+  float neq[Q], gp[Q];
+  non_equilibrium(Geq(mo, kScale), g, neq);
+  float tau, om;
+  site_rate<S, K>(a, neq, s, tau, om);
+  relax(g, neq, K == kTRT, om, (float)a.omega_minus, gp);
+  S* o = static_cast<S*>(m.fout) + s;
+  Store<S>::st(o, gp[0]);
 #pragma unroll
-  for (int i = 0; i < Q; i++) out[i] = gp[i] = collide_one_f<K>(a, g, fneq, om, i);
-  int io = -1;
-  if (im) {
-    io = __ldg(G.io + gi);
+  for (int i = 1; i < Q; i++)
+    if (WALL != kGZS || ((keep >> (i - 1)) & 1u)) Store<S>::st(o + (int64_t)i * a.np, gp[i]);
+  const uint32_t im = l.iolet;
+  if (IO && im) {
+    const int io = __ldg(G.io + gi);
     const IoletDev& I = a.iolets[io];
     const double pos[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
+    const float r = kScale + mo.D, rho = 1.0f + mo.D * (1.0f / kScale);
+    const float ux = mo.mx / r, uy = mo.my / r, uz = mo.mz / r;
 #pragma unroll
     for (int d = 1; d < Q; d++) {
       if (!((im >> (d - 1)) & 1u)) continue;
@@ -425,101 +504,104 @@ __device__ __forceinline__ void general_site_m(const StepArgs& a, const MixArgs&
           w[0] = w[1] = w[2] = 0.0f;
         }
         const float corr = 2.0f * wf(d) * rho * (w[0] * cx(d) + w[1] * cy(d) + w[2] * cz(d)) * 3.0f;
-        v = gp[d] - corr;
+        v = gp[d] * (1.0f / kScale) - corr;
       } else {
         const double rb = a.dens_row[io];
         const float drb = (float)(rb - 1.0);
         const float rbf = (float)rb;
         const float nx = (float)I.nrm_f[0], ny = (float)I.nrm_f[1], nz = (float)I.nrm_f[2];
         const float comp = ux * nx + uy * ny + uz * nz;
-        const GeqF gq(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf);
+        const Geq gq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f);
         v = gq(inv(d));
       }
       m.gout[(int64_t)(d - 1) * G.G + gi] = v;
     }
-  }
-  if (WALL == kGZS && wm) {
-#pragma unroll
-    for (int d = 1; d < Q; d++) {
-      if (!((wm >> (d - 1)) & 1u)) continue;
-      const int i = inv(d);
-      const float q = __ldg(G.q + (int64_t)(d - 1) * G.G + gi);
-      const float fac = 1.0f - 1.0f / q;
-      float mw0 = mx * fac, mw1 = my * fac, mw2 = mz * fac;
-      float fnw_i = fneq[i], fnw_d = fneq[d];
-      bool sbb = false;
-      if (q < 0.75f) {
-        if ((im >> (i - 1)) & 1u) {
-          const IoletDev& I = a.iolets[io];
-          if (!is_velocity_iolet(I.kind)) {
-            sbb = true;
-          } else {
-            const double p3[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
-            float nv[3];
-            if (!link_velocity_f(a, I, io, gi, i, false, p3, nv)) {
-              atomicOr(a.status, kStatusIoletRadius);
-              nv[0] = nv[1] = nv[2] = 0.0f;
-            }
-            const float k2 = (1.0f - q) * rho * (q - 1.0f) / (q + 1.0f);
-            mw0 = q * mw0 + k2 * nv[0];
-            mw1 = q * mw1 + k2 * nv[1];
-            mw2 = q * mw2 + k2 * nv[2];
-          }
-        } else if ((wm >> (i - 1)) & 1u) {
-          sbb = true;
-        } else {
-          const int grun = __ldg(G.run + gi);
-          const int nb = grun >= 0 ? s + __ldg(a.run_off + 20 * grun + d) : __ldg(G.src + (int64_t)(d - 1) * G.G + gi);
-          float gn[Q];
-          gather_any_m<S, WALL, GATHER>(a, m, nb, gn);
-          float dn, mnx, mny, mnz;
-          moments_g(gn, dn, mnx, mny, mnz);
-          const float rn = 1.0f + dn;
-          const GeqF gqn(dn, mnx, mny, mnz);
-          const float k2 = (1.0f - q) * rho * (q - 1.0f) / (q + 1.0f) / rn;
-          mw0 = q * mw0 + k2 * mnx;
-          mw1 = q * mw1 + k2 * mny;
-          mw2 = q * mw2 + k2 * mnz;
-          fnw_i = q * fnw_i + (1.0f - q) * (gn[i] - gqn(i));
-          fnw_d = q * fnw_d + (1.0f - q) * (gn[d] - gqn(d));
-        }
-      }
-      if (sbb) continue;
-      const GeqF gw(drho, mw0, mw1, mw2);
-      const float gw_i = gw(i) + fnw_i;
-      float v;
-      if (K == kTRT) {
-        const float sym = 0.5f * (float)a.omega * (fnw_i + fnw_d);
-        const float asym = 0.5f * (float)a.omega_minus * (fnw_i - fnw_d);
-        v = gw_i + sym + asym;
-      } else {
-        v = gw_i + fnw_i * om;
-      }
-      out[d] = v;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < Q; i++) Store<S>::store(m.fout, (int64_t)i * a.np + s, out[i]);
-  const int cpl = im ? __ldg(G.cpl + gi) : -1;
-  if (cpl >= 0) {
-    const IoletDev& I = a.iolets[io];
-    a.cpl_buf[cpl] = (double)ux * (-I.nrm[0]) + (double)uy * (-I.nrm[1]) + (double)uz * (-I.nrm[2]);
+    const int cpl = __ldg(G.cpl + gi);
+    if (cpl >= 0) a.cpl_buf[cpl] = (double)ux * (-I.nrm[0]) + (double)uy * (-I.nrm[1]) + (double)uz * (-I.nrm[2]);
   }
   if (MACRO) {
-    a.rho[s] = (double)rho;
-    a.u[s] = (double)ux;
-    a.u[a.np + s] = (double)uy;
-    a.u[2 * a.np + s] = (double)uz;
-    if (wm) {
-      const float nor[3] = {__ldg(G.nrm + gi), __ldg(G.nrm + G.G + gi), __ldg(G.nrm + 2 * G.G + gi)};
-      a.wss[s] = wss_mag_f(tau, gp, g, nor);
-    } else {
-      a.wss[s] = kNoValue;
-    }
-    if (a.pi) store_pi_f(a, s, tau, gp, g);
+    const float nor[3] = {__ldg(G.nrm + gi), __ldg(G.nrm + G.G + gi), __ldg(G.nrm + 2 * G.G + gi)};
+    store_macro<S>(a, s, mo, tau, gp, g, l.wall != 0u, nor);
   }
 }
 
-// Pre-collision f (FP64, AoS, reference order) from the shifted storage.
+// v[i] for an index known at run time only, without an indexed array.
+__device__ __forceinline__ float pick_m(const float* v, int i) {
+  float x = v[1];
+#pragma unroll
+  for (int k = 2; k < Q; k++) x = k == i ? v[k] : x;
+  return x;
+}
+
+// Equilibrium of a direction known at run time only.
+__device__ __forceinline__ float geq_at(const Geq& c, int i) {
+  const float w = i < 7 ? wf(1) : wf(7);
+  const float e = (float)cx(i) * c.mx + (float)cy(i) * c.my + (float)cz(i) * c.mz;
+  return vfma(w, e, vfma(w * c.nh * e, e, w * c.t1));
+}
+
+// The virtual-node value of entry k of the GZS link list, one thread per link
+// (gzs_link_f64 in FP32 on the stored scale).
+template <class S, int K, bool GATHER, bool PDL = false>
+__device__ __forceinline__ void gzs_link_m(const StepArgs& a, const MixArgs& m, int k) {
+  const GeneralDev& G = a.gen;
+  constexpr float kScale = Store<S>::kScale;
+  const bool live = k < a.gzs_n;
+  int gi = 0, d = 1, s = 0, i = 0, nb = 0;
+  uint32_t im = 0;
+  float q = 1.0f;
+  bool extrapolate = false;
+  if (live) {
+    gi = __ldg(a.gzs_rec + k);
+    d = __ldg(a.gzs_dir + k);
+    i = (d & 1) ? d + 1 : d - 1;
+    s = __ldg(G.site + gi);
+    im = __ldg(G.iolet + gi);
+    const int run = __ldg(G.run + gi);
+    q = __ldg(G.q + (int64_t)(d - 1) * G.G + gi);
+    extrapolate = q < 0.75f && !((im >> (i - 1)) & 1u);
+    nb = s;
+    if (extrapolate) nb = run >= 0 ? s + __ldg(a.run_off + 20 * run + d) : __ldg(G.src + (int64_t)(d - 1) * G.G + gi);
+  }
+  if (PDL) wait_previous_step();
+  if (!live) return;
+  float g[Q], gn[Q];
+  gather_any_m<S, kGZS, GATHER>(a, m, s, g);
+  gather_any_m<S, kGZS, GATHER>(a, m, nb, gn);
+  const Moments mo(g);
+  const Geq geq(mo, kScale);
+  const float rho = kScale + mo.D;
+  float fi = pick_m(g, i) - geq_at(geq, i), fd = pick_m(g, d) - geq_at(geq, d);
+  const float fac = 1.0f - 1.0f / q;
+  float mw0 = mo.mx * fac, mw1 = mo.my * fac, mw2 = mo.mz * fac;
+  if (extrapolate) {
+    const Moments mn(gn);
+    const Geq geqn(mn, kScale);
+    const float k2 = (1.0f - q) * rho * (q - 1.0f) / (q + 1.0f) / (kScale + mn.D);
+    mw0 = q * mw0 + k2 * mn.mx;
+    mw1 = q * mw1 + k2 * mn.my;
+    mw2 = q * mw2 + k2 * mn.mz;
+    fi = q * fi + (1.0f - q) * (pick_m(gn, i) - geq_at(geqn, i));
+    fd = q * fd + (1.0f - q) * (pick_m(gn, d) - geq_at(geqn, d));
+  } else if (q < 0.75f) {  // behind the site: a velocity iolet
+    const int io = __ldg(G.io + gi);
+    const double p3[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
+    float nv[3];
+    if (!link_velocity_f(a, a.iolets[io], io, gi, i, false, p3, nv)) {
+      atomicOr(a.status, kStatusIoletRadius);
+      nv[0] = nv[1] = nv[2] = 0.0f;
+    }
+    const float k2 = (1.0f - q) * rho * (q - 1.0f) / (q + 1.0f);
+    mw0 = q * mw0 + k2 * nv[0];
+    mw1 = q * mw1 + k2 * nv[1];
+    mw2 = q * mw2 + k2 * nv[2];
+  }
+  const float gw_i = geq_at(Geq(Moments(mo.D, mw0, mw1, mw2), kScale), i) + fi;
+  float v;
+  if (K == kTRT) v = gw_i + 0.5f * (float)a.omega * (fi + fd) + 0.5f * (float)a.omega_minus * (fi - fd);
+  else v = gw_i + fi * (float)a.omega;
+  Store<S>::st(static_cast<S*>(m.fout) + (int64_t)d * a.np + s, v);
+}
+
 }  // namespace
 }  // namespace hb

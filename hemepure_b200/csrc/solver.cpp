@@ -111,18 +111,15 @@ Solver::Solver(LatticeTables tables, const hb_params& params, const hb_options& 
     omega_minus_ = -1.0 / tau_minus;
   }
   check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-  // The latency-bound boundary kernel runs on the side stream at the highest
-  // priority, so its blocks are dispatched ahead of the bulk kernel's queued ones
-  // (4M-site pipe: FP32 step 29.3k -> 30.3k MLUPS; FP64 unchanged).
+  // The Windkessel update and the iolet records run on the side stream at the
+  // highest priority, so their few blocks are not queued behind the step's.
   int prio_lo = 0, prio_hi = 0;
   check(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi), "cudaDeviceGetStreamPriorityRange");
   check(cudaStreamCreateWithPriority(&side_, cudaStreamNonBlocking, prio_hi), "cudaStreamCreate");
-  check(cudaStreamCreateWithPriority(&side2_, cudaStreamNonBlocking, prio_hi), "cudaStreamCreate");
   check(cudaEventCreate(&ev0_), "cudaEventCreate");
   check(cudaEventCreate(&ev1_), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming), "cudaEventCreate");
-  check(cudaEventCreateWithFlags(&join2_, cudaEventDisableTiming), "cudaEventCreate");
   upload();
 }
 
@@ -130,14 +127,11 @@ Solver::~Solver() {
   if (stream_) cudaStreamSynchronize(stream_);
   if (xev_) cudaEventDestroy(xev_);
   if (side_) cudaStreamSynchronize(side_);
-  if (side2_) cudaStreamSynchronize(side2_);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   if (fork_) cudaEventDestroy(fork_);
   if (join_) cudaEventDestroy(join_);
-  if (join2_) cudaEventDestroy(join2_);
   if (side_) cudaStreamDestroy(side_);
-  if (side2_) cudaStreamDestroy(side2_);
   if (stream_) cudaStreamDestroy(stream_);
   if (status_host_) cudaFreeHost(status_host_);
   if (host_rows_) cudaFreeHost(host_rows_);
@@ -173,7 +167,13 @@ void Solver::upload() {
   upload_vec(g_wall_, L_.g_wall, tot);
   upload_vec(g_iolet_, L_.g_iolet, tot);
   upload_vec(g_src_, L_.g_src, tot);
-  upload_vec(g_q_, L_.g_q, tot);
+  if (mixed() && opt_.wall == kBFL) {
+    std::vector<float> coef(L_.g_q);
+    for (float& q : coef) q = bfl_coefficient(q);
+    upload_vec(g_q_, coef, tot);
+  } else {
+    upload_vec(g_q_, L_.g_q, tot);
+  }
   upload_vec(g_nrm_, L_.g_nrm, tot);
   upload_vec(g_io_, L_.g_io, tot);
   upload_vec(g_cpl_, L_.g_cpl, tot);
@@ -491,8 +491,12 @@ void Solver::set_iolet_densities(const double* inlets, int n_inlets, const doubl
 
 void Solver::request_comms() {
   if (!phase_open_) row_ = density_row(t_step_, 1);
-  launch_wk3_begin(wk3_.as<WK3Dev>(), nwk3_, cpl_buf_.as<double>(), dens_.as<double>() + (size_t)row_ * kRowStride, stream_);
+  launch_wk3(stream_);
   phase_open_ = true;
+}
+
+void Solver::launch_wk3(cudaStream_t st) {
+  launch_wk3_begin(wk3_.as<WK3Dev>(), nwk3_, cpl_buf_.as<double>(), dens_.as<double>() + (size_t)row_ * kRowStride, st);
 }
 
 void Solver::pre_receive(bool macro, int which, bool stress) {
@@ -505,28 +509,17 @@ void Solver::pre_receive(bool macro, int which, bool stress) {
   }
   StepArgs a = args();
   a.pi = stress ? pi_.as<double>() : nullptr;
-  // Boundary records with iolet links run in their own kernel on a second side
-  // stream, beside those without (independent records, disjoint slots).  4M
-  // pipe, whole step: FP64 0.2140 -> 0.2136 ms, FP32 0.1208 -> 0.1190 ms, FP16
-  // 0.0963 -> 0.0903 ms.  Their few blocks are launched first, so they are not
-  // queued behind the wall records' four waves (boundary work alone: FP64
-  // 0.0430 -> 0.0390 ms, FP16 0.0383 -> 0.0317 ms).
-  const bool split = L_.kind_start[2] > 0 && L_.kind_start[2] < L_.G;
-  if ((which & kLaunchBoundary) && L_.G > 0) {
-    // The boundary kernels are latency-bound and the bulk kernel bandwidth-bound:
-    // run them side by side, all after the Windkessel update.
+  if (wk_beside_) {
+    // The Windkessel update (one block per iolet adding its sites' flows in order)
+    // and the records that read its density run on the side stream, beside the rest.
     check(cudaEventRecord(fork_, stream_), "fork");
-    if (split) {
-      check(cudaStreamWaitEvent(side2_, fork_, 0), "fork");
-      launch(a, macro, kLaunchIoletRecords, side2_);
-      check(cudaEventRecord(join2_, side2_), "join");
-    }
     check(cudaStreamWaitEvent(side_, fork_, 0), "fork");
-    launch(a, macro, split ? kLaunchWallRecords : kLaunchBoundary, side_);
+    launch_wk3(side_);
+    launch(a, macro, kLaunchIoletRecords, side_);
     check(cudaEventRecord(join_, side_), "join");
-    if (which & kLaunchBulk) launch(a, macro, kLaunchBulk, stream_);
+    launch(a, macro, which & ~kLaunchIoletRecords, stream_);
     check(cudaStreamWaitEvent(stream_, join_, 0), "join");
-    if (split) check(cudaStreamWaitEvent(stream_, join2_, 0), "join");
+    wk_beside_ = false;
   } else {
     launch(a, macro, which, stream_);
   }
@@ -535,9 +528,16 @@ void Solver::pre_receive(bool macro, int which, bool stress) {
   phase_stress_ = stress;
 }
 
+// Kernels of one step: one for a steady-state step (two with the iolet records
+// beside it), else one per kind of work.
+int Solver::step_launches(bool macro) const {
+  if (direct_ || macro) return 1 + (L_.G > 0 ? 1 : 0) + (gzs_n_ > 0 ? 1 : 0);
+  return 1 + (wk_beside_ && L_.G > L_.kind_start[2] ? 1 : 0);
+}
+
 void Solver::launch(const StepArgs& a, bool macro, int which, cudaStream_t st) {
   if (!mixed()) {
-    launch_step_f64(a, opt_.kernel, opt_.wall, !direct_, macro, which, 256, 128, st);
+    launch_step_f64(a, opt_.kernel, opt_.wall, !direct_, macro, which, st);
   } else {
     launch_step_mixed(a, opt_.precision, f_[cur_].p, f_[1 - cur_].p, ghost_[cur_].as<float>(), ghost_[1 - cur_].as<float>(),
                       opt_.kernel, opt_.wall, !direct_, macro, which, st);
@@ -584,19 +584,16 @@ int Solver::step(int64_t nsteps, uint32_t flags) {
   if (shard_ && nsteps > 1)
     throw Error{HB_ERR_ARG, "a shard advances one step per call: its halo is exchanged between steps"};
   int64_t launches = 0;
-  // The boundary records without and with iolet links are two kernels.
-  const int boundary_launches =
-      L_.G == 0 ? 0 : (L_.kind_start[2] > 0 ? 1 : 0) + (L_.G > L_.kind_start[2] ? 1 : 0);
-  const int per_step = (nwk3_ ? 1 : 0) + (L_.n > 0 ? 1 : 0) + boundary_launches;
   check(cudaEventRecord(ev0_, stream_), "event");
   for (int64_t j = 0; j < nsteps; j++) {
     row_ = density_row(t_step_, nsteps - j);
     phase_open_ = true;
-    launch_wk3_begin(wk3_.as<WK3Dev>(), nwk3_, cpl_buf_.as<double>(), dens_.as<double>() + (size_t)row_ * kRowStride, stream_);
     const bool macro = (flags & HB_STEP_MACRO) && (j == nsteps - 1);
-    pre_receive(macro, 3, (flags & HB_STEP_STRESS) != 0);
+    wk_beside_ = nwk3_ > 0 && !direct_ && !macro;  // the other forms launch every record at once
+    if (!wk_beside_) launch_wk3(stream_);
+    launches += (nwk3_ ? 1 : 0) + step_launches(macro);
+    pre_receive(macro, kLaunchAll, (flags & HB_STEP_STRESS) != 0);
     end_iteration();
-    launches += per_step;
   }
   check(cudaEventRecord(ev1_, stream_), "event");
   const int st = read_status();
@@ -621,15 +618,15 @@ int Solver::profile(int64_t nsteps, double ms[3]) {
       {
         row_ = density_row(t_step_, nsteps - j);
         phase_open_ = true;
-        launch_wk3_begin(wk3_.as<WK3Dev>(), nwk3_, cpl_buf_.as<double>(), dens_.as<double>() + (size_t)row_ * kRowStride, stream_);
+        launch_wk3(stream_);
         check(cudaEventRecord(e[0], stream_), "event");
         if (pass == 0) {
-          pre_receive(false, 3);
+          pre_receive(false, kLaunchAll);
           check(cudaEventRecord(e[1], stream_), "event");
         } else {
-          pre_receive(false, 1);
+          pre_receive(false, kLaunchBulk);
           check(cudaEventRecord(e[1], stream_), "event");
-          pre_receive(false, 2);
+          pre_receive(false, kLaunchBoundary);
         }
         check(cudaEventRecord(e[2], stream_), "event");
         end_iteration();

@@ -40,7 +40,7 @@ class Solver {
   // lb::LBM phases.
   void request_comms();
   // `stress` (with `macro`) also stores the momentum flux tensor for the stress caches.
-  void pre_receive(bool macro, int which = 3, bool stress = false);
+  void pre_receive(bool macro, int which = kLaunchAll, bool stress = false);
   void end_iteration();
   int step(int64_t n, uint32_t flags);
   // `n` steps with CUDA events around each launch: ms[0] plain bulk kernel,
@@ -124,6 +124,8 @@ class Solver {
   bool mixed() const { return opt_.precision != HB_STORE_FP64; }
   size_t elem_bytes() const { return opt_.precision == HB_STORE_FP64 ? 8 : (opt_.precision == HB_STORE_FP32 ? 4 : 2); }
   void launch(const StepArgs& a, bool macro, int which, cudaStream_t st);
+  void launch_wk3(cudaStream_t st);
+  int step_launches(bool macro) const;
   void to_aos(bool use_prev, double* dev_aos);
 
   LatticeTables t_;
@@ -132,10 +134,9 @@ class Solver {
   hb_options opt_;
   Layout L_;
   cudaStream_t stream_ = nullptr;
-  cudaStream_t side_ = nullptr;   // boundary kernel, concurrent with the bulk kernel
+  cudaStream_t side_ = nullptr;   // Windkessel update and iolet records, beside the other sites
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
-  cudaStream_t side2_ = nullptr;  // the boundary records with iolet links, beside the others
-  cudaEvent_t fork_ = nullptr, join_ = nullptr, join2_ = nullptr;
+  cudaEvent_t fork_ = nullptr, join_ = nullptr;
 
   DeviceBuffer f_[2];
   DeviceBuffer ghost_[2];         // iolet ghost values, paired with f_
@@ -164,6 +165,7 @@ class Solver {
   bool dens_override_ = false;
   double dens_override_v_[32] = {};  // inlets 0-15, outlets 16-31
   int nwk3_ = 0;
+  bool wk_beside_ = false;        // the step being issued runs its Windkessel update on side_
   bool macro_valid_ = false;
   bool phase_open_ = false;
   bool phase_macro_ = false;
