@@ -76,6 +76,10 @@ struct StepArgs {
   const int* run_off;
   const int* run_po;      // [runs][20] plane offsets i * np + run_off[run][i] (shifted forms' bulk kernel), or null
   GeneralDev gen;
+  // Iolet links, listed as the GZS links below.
+  const int* iol_rec;
+  const uint8_t* iol_dir;
+  int iol_n;
   // GZS wall links with a virtual node (GZS walls only): the record and the
   // direction of each, 32 records' links of one direction after the other.
   const int* gzs_rec;

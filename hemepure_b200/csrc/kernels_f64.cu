@@ -32,8 +32,9 @@ namespace {
 constexpr int kStepBlocksPerSM = 4;
 
 // One steady-state time step (gathering, no outputs) in one launch: the grid's
-// blocks of kStepBlock threads take boundary records with iolet links, GZS wall
-// links, boundary records without iolet links and plain bulk sites (StepTiles).
+// blocks of kStepBlock threads take iolet links, boundary records with such links,
+// GZS wall links, boundary records without iolet links and plain bulk sites
+// (StepTiles).
 // The bulk blocks are bound by HBM bandwidth and the boundary blocks by latency,
 // so the wall-record blocks are spread evenly among the bulk blocks instead of
 // running ahead of them, and the long iolet and link blocks come first.  The
@@ -47,6 +48,11 @@ constexpr int kStepBlocksPerSM = 4;
 template <int K, int WALL>
 __global__ void __launch_bounds__(kStepBlock, kStepBlocksPerSM) k_step(const StepArgs a, const StepTiles t) {
   int b = blockIdx.x;
+  if (b < t.links) {
+    iolet_link_f64<K, WALL, true, true>(a, b * kStepBlock + threadIdx.x);
+    return;
+  }
+  b -= t.links;
   if (b < t.io) {
     const int g = t.io_first + b * kStepBlock + threadIdx.x;
     general_site_f64<K, WALL, true, false, true, true>(a, g, g < a.gen.G);
@@ -101,6 +107,11 @@ __global__ void __launch_bounds__(128) k_general(const StepArgs a) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.gen.G) return;
   general_site_f64<K, WALL, GATHER, MACRO>(a, g);
+}
+
+template <int K, int WALL, bool GATHER>
+__global__ void __launch_bounds__(128) k_iolets(const StepArgs a) {
+  iolet_link_f64<K, WALL, GATHER>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 template <int K, bool GATHER>
@@ -321,6 +332,7 @@ template <int K, int WALL, bool GATHER, bool MACRO>
 void launch_parts(const StepArgs& a, cudaStream_t st) {
   if (a.n > 0) k_bulk<K, GATHER, MACRO><<<(a.n + 255) / 256, 256, 0, st>>>(a);
   if (a.gen.G > 0) k_general<K, WALL, GATHER, MACRO><<<(a.gen.G + 127) / 128, 128, 0, st>>>(a);
+  if (a.iol_n > 0) k_iolets<K, WALL, GATHER><<<(a.iol_n + 127) / 128, 128, 0, st>>>(a);
   if constexpr (has_gzs(K))
     if (a.gzs_n > 0) k_gzs<K, GATHER><<<(a.gzs_n + 127) / 128, 128, 0, st>>>(a);
 }

@@ -16,8 +16,9 @@
 namespace hb {
 namespace {
 
-template <class S>
-constexpr int kMixedBlocksPerSM = sizeof(S) == 2 ? 8 : 6;
+// 64 registers.  4M-site pipe FP32: five blocks 143.5 us a step, six 128.3, seven
+// 122.7, eight 120.7; FP16: six 91, eight 85.4, ten 102.
+constexpr int kMixedBlocksPerSM = 8;
 
 // One steady-state time step in one launch (k_step of kernels_f64.cu): boundary
 // records with iolet links, GZS wall links, then the other boundary records
@@ -29,8 +30,13 @@ constexpr int kMixedBlocksPerSM = sizeof(S) == 2 ? 8 : 6;
 // take 102 registers (FP32 127, FP16 93 us), and the bulk sites in a kernel of their
 // own at 40 registers beside the boundary records measure 121 and 90.
 template <class S, int K, int WALL>
-__global__ void __launch_bounds__(kStepBlock, kMixedBlocksPerSM<S>) k_step_m(const StepArgs a, const MixArgs m, const StepTiles t) {
+__global__ void __launch_bounds__(kStepBlock, kMixedBlocksPerSM) k_step_m(const StepArgs a, const MixArgs m, const StepTiles t) {
   int b = blockIdx.x;
+  if (b < t.links) {
+    iolet_link_m<S, K, WALL, true, true>(a, m, b * kStepBlock + threadIdx.x);
+    return;
+  }
+  b -= t.links;
   if (b < t.io) {
     const int g = t.io_first + b * kStepBlock + threadIdx.x;
     general_site_m<S, K, WALL, true, false, true, true>(a, m, g, g < a.gen.G);
@@ -90,6 +96,11 @@ __global__ void __launch_bounds__(128) k_general_m(const StepArgs a, const MixAr
   general_site_m<S, K, WALL, GATHER, MACRO>(a, m, gi);
 }
 
+template <class S, int K, int WALL, bool GATHER>
+__global__ void __launch_bounds__(128) k_iolets_m(const StepArgs a, const MixArgs m) {
+  iolet_link_m<S, K, WALL, GATHER>(a, m, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 template <class S, int K, bool GATHER>
 __global__ void __launch_bounds__(128) k_gzs_m(const StepArgs a, const MixArgs m) {
   gzs_link_m<S, K, GATHER>(a, m, blockIdx.x * blockDim.x + threadIdx.x);
@@ -122,6 +133,7 @@ template <class S, int K, int WALL, bool GATHER, bool MACRO>
 void launch_parts(const StepArgs& a, const MixArgs& m, cudaStream_t st) {
   if (a.n > 0) k_bulk_m<S, K, GATHER, MACRO><<<(a.n + 255) / 256, 256, 0, st>>>(a, m);
   if (a.gen.G > 0) k_general_m<S, K, WALL, GATHER, MACRO><<<(a.gen.G + 127) / 128, 128, 0, st>>>(a, m);
+  if (a.iol_n > 0) k_iolets_m<S, K, WALL, GATHER><<<(a.iol_n + 127) / 128, 128, 0, st>>>(a, m);
   if constexpr (WALL == kGZS)
     if (a.gzs_n > 0) k_gzs_m<S, K, GATHER><<<(a.gzs_n + 127) / 128, 128, 0, st>>>(a, m);
 }
@@ -129,7 +141,7 @@ void launch_parts(const StepArgs& a, const MixArgs& m, cudaStream_t st) {
 template <class S, int K, int WALL>
 void launch_m2(const StepArgs& a, const MixArgs& m, bool gather, bool macro, int which, cudaStream_t st) {
   if (gather && !macro) {
-    const StepTiles t = step_tiles(a, which, kMixedBlocksPerSM<S>);
+    const StepTiles t = step_tiles(a, which, kMixedBlocksPerSM);
     launch_dependent(k_step_m<S, K, WALL>, t.blocks(), st, a, m, t);
   } else if (gather) {
     launch_parts<S, K, WALL, true, true>(a, m, st);

@@ -444,8 +444,9 @@ __device__ __forceinline__ void bulk_site_m(const StepArgs& a, const MixArgs& m,
 }
 
 // One general site gi (`live` false: no record; the thread only waits for the
-// previous step).  A GZS wall link's virtual-node value comes from gzs_link_m, so
-// its slot is not stored here.
+// previous step).  The ghost values of its iolet links come from iolet_link_m, and
+// a GZS wall link's virtual-node value from gzs_link_m, so that link's slot is not
+// stored here.
 template <class S, int K, int WALL, bool GATHER, bool MACRO, bool IO = true, bool PDL = false>
 __device__ __forceinline__ void general_site_m(const StepArgs& a, const MixArgs& m, int gi, bool live = true) {
   const GeneralDev& G = a.gen;
@@ -486,38 +487,14 @@ __device__ __forceinline__ void general_site_m(const StepArgs& a, const MixArgs&
 #pragma unroll
   for (int i = 1; i < Q; i++)
     if (WALL != kGZS || ((keep >> (i - 1)) & 1u)) Store<S>::st(o + (int64_t)i * a.np, gp[i]);
-  const uint32_t im = l.iolet;
-  if (IO && im) {
-    const int io = __ldg(G.io + gi);
-    const IoletDev& I = a.iolets[io];
-    const double pos[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
-    const float r = kScale + mo.D, rho = 1.0f + mo.D * (1.0f / kScale);
-    const float ux = mo.mx / r, uy = mo.my / r, uz = mo.mz / r;
-#pragma unroll
-    for (int d = 1; d < Q; d++) {
-      if (!((im >> (d - 1)) & 1u)) continue;
-      float v;
-      if (is_velocity_iolet(I.kind)) {
-        float w[3];
-        if (!link_velocity_f(a, I, io, gi, d, true, pos, w)) {
-          atomicOr(a.status, kStatusIoletRadius);
-          w[0] = w[1] = w[2] = 0.0f;
-        }
-        const float corr = 2.0f * wf(d) * rho * (w[0] * cx(d) + w[1] * cy(d) + w[2] * cz(d)) * 3.0f;
-        v = gp[d] * (1.0f / kScale) - corr;
-      } else {
-        const double rb = a.dens_row[io];
-        const float drb = (float)(rb - 1.0);
-        const float rbf = (float)rb;
-        const float nx = (float)I.nrm_f[0], ny = (float)I.nrm_f[1], nz = (float)I.nrm_f[2];
-        const float comp = ux * nx + uy * ny + uz * nz;
-        const Geq gq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f);
-        v = gq(inv(d));
-      }
-      m.gout[(int64_t)(d - 1) * G.G + gi] = v;
-    }
+  if (IO && l.iolet) {
     const int cpl = __ldg(G.cpl + gi);
-    if (cpl >= 0) a.cpl_buf[cpl] = (double)ux * (-I.nrm[0]) + (double)uy * (-I.nrm[1]) + (double)uz * (-I.nrm[2]);
+    if (cpl >= 0) {
+      const IoletDev& I = a.iolets[__ldg(G.io + gi)];
+      const float r = kScale + mo.D;
+      const float ux = mo.mx / r, uy = mo.my / r, uz = mo.mz / r;
+      a.cpl_buf[cpl] = (double)ux * (-I.nrm[0]) + (double)uy * (-I.nrm[1]) + (double)uz * (-I.nrm[2]);
+    }
   }
   if (MACRO) {
     const float nor[3] = {__ldg(G.nrm + gi), __ldg(G.nrm + G.G + gi), __ldg(G.nrm + 2 * G.G + gi)};
@@ -601,6 +578,69 @@ __device__ __forceinline__ void gzs_link_m(const StepArgs& a, const MixArgs& m, 
   if (K == kTRT) v = gw_i + 0.5f * (float)a.omega * (fi + fd) + 0.5f * (float)a.omega_minus * (fi - fd);
   else v = gw_i + fi * (float)a.omega;
   Store<S>::st(static_cast<S*>(m.fout) + (int64_t)d * a.np + s, v);
+}
+
+// The ghost value of entry k of the iolet link list, one thread per link
+// (iolet_link_f64 in FP32; the imposed velocity and density in FP64).
+template <class S, int K, int WALL, bool GATHER, bool PDL = false>
+__device__ __forceinline__ void iolet_link_m(const StepArgs& a, const MixArgs& m, int k) {
+  const GeneralDev& G = a.gen;
+  constexpr float kScale = Store<S>::kScale;
+  const bool live = k < a.iol_n;
+  const int gi = live ? __ldg(a.iol_rec + k) : 0, d = live ? __ldg(a.iol_dir + k) : 1;
+  LinksM l{0u, 0u, 0, gi};
+  int s = 0, src[18];
+  if (live) {
+    s = __ldg(G.site + gi);
+    l.wall = __ldg(G.wall + gi);
+    l.iolet = __ldg(G.iolet + gi);
+    l.run = __ldg(G.run + gi);
+    if (GATHER) load_sources_m(a, l, s, src);
+  }
+  if (PDL) wait_previous_step();
+  if (!live) return;
+  float g[Q];
+  if (GATHER) gather_links_m<S>(a, m, l, s, src, WALL == kBFL, g);
+  else {
+    const S* p = static_cast<const S*>(m.fin) + s;
+#pragma unroll
+    for (int i = 0; i < Q; i++) g[i] = Store<S>::ld(p + (int64_t)i * a.np);
+  }
+  const Moments mo(g);
+  const int io = __ldg(G.io + gi), i = (d & 1) ? d + 1 : d - 1;
+  const IoletDev& I = a.iolets[io];
+  float v;
+  if (is_velocity_iolet(I.kind)) {
+    float neq[Q], tau, om, w[3];
+    non_equilibrium(Geq(mo, kScale), g, neq);
+    site_rate<S, K>(a, neq, s, tau, om);
+    const float nd = pick_m(neq, d);
+    float post;
+    if (K == kTRT) {
+      const float ni = pick_m(neq, i);
+      post = vfma(0.5f * (float)a.omega_minus, vsub(nd, ni), vfma(0.5f * om, vadd(nd, ni), pick_m(g, d)));
+    } else {
+      post = vfma(om, nd, pick_m(g, d));
+    }
+    const double pos[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
+    if (!link_velocity_f(a, I, io, gi, d, true, pos, w)) {
+      atomicOr(a.status, kStatusIoletRadius);
+      w[0] = w[1] = w[2] = 0.0f;
+    }
+    const float rho = 1.0f + mo.D * (1.0f / kScale);
+    const float corr = 2.0f * (d < 7 ? wf(1) : wf(7)) * rho * (w[0] * cx(d) + w[1] * cy(d) + w[2] * cz(d)) * 3.0f;
+    v = post * (1.0f / kScale) - corr;
+  } else {
+    const float r = kScale + mo.D;
+    const float ux = mo.mx / r, uy = mo.my / r, uz = mo.mz / r;
+    const double rb = a.dens_row[io];
+    const float drb = (float)(rb - 1.0);
+    const float rbf = (float)rb;
+    const float nx = (float)I.nrm_f[0], ny = (float)I.nrm_f[1], nz = (float)I.nrm_f[2];
+    const float comp = ux * nx + uy * ny + uz * nz;
+    v = geq_at(Geq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f), i);
+  }
+  m.gout[(int64_t)(d - 1) * G.G + gi] = v;
 }
 
 }  // namespace

@@ -67,6 +67,30 @@ void upload_vec(DeviceBuffer& b, const std::vector<T>& v, int64_t& total) {
   total += (int64_t)b.bytes;
 }
 
+// The links of `mask` as a list: 32 records' links of one direction after the
+// other, so a warp's records are neighbours and its direction mostly one.
+int upload_links(const std::vector<uint32_t>& mask, DeviceBuffer& rec, DeviceBuffer& dir, int64_t& total) {
+  std::vector<int> r;
+  std::vector<uint8_t> d;
+  const int G = (int)mask.size();
+  for (int g0 = 0; g0 < G; g0 += 32) {
+    const int g1 = std::min(G, g0 + 32);
+    uint32_t any = 0;
+    for (int g = g0; g < g1; g++) any |= mask[g];
+    for (; any; any &= any - 1) {
+      const int bit = __builtin_ctz(any);
+      for (int g = g0; g < g1; g++)
+        if ((mask[g] >> bit) & 1u) {
+          r.push_back(g);
+          d.push_back((uint8_t)(bit + 1));
+        }
+    }
+  }
+  upload_vec(rec, r, total);
+  upload_vec(dir, d, total);
+  return (int)r.size();
+}
+
 }  // namespace
 
 void validate_case(const hb_params& p, const hb_options& o) {
@@ -178,6 +202,7 @@ void Solver::upload() {
   upload_vec(g_io_, L_.g_io, tot);
   upload_vec(g_cpl_, L_.g_cpl, tot);
   upload_vec(g_xyz_, L_.g_xyz, tot);
+  iol_n_ = upload_links(L_.g_iolet, iol_rec_, iol_dir_, tot);
   // GZS wall links: all but those that bounce back (q < 3/4 with a wall or a
   // pressure iolet behind the site, src/lb/streamers/GuoZhengShiDelegate.h:127-293).
   if (opt_.wall == kGZS) {
@@ -195,19 +220,8 @@ void Solver::upload() {
         }
         mask[g] |= 1u << (d - 1);
       }
-    std::vector<int> rec;
-    std::vector<uint8_t> dir;
-    for (int g0 = 0; g0 < L_.G; g0 += 32)
-      for (int d = 1; d < Q; d++)
-        for (int g = g0; g < std::min(L_.G, g0 + 32); g++)
-          if ((mask[g] >> (d - 1)) & 1u) {
-            rec.push_back(g);
-            dir.push_back((uint8_t)d);
-          }
-    gzs_n_ = (int)rec.size();
     upload_vec(g_gzs_, mask, tot);
-    upload_vec(gzs_rec_, rec, tot);
-    upload_vec(gzs_dir_, dir, tot);
+    gzs_n_ = upload_links(mask, gzs_rec_, gzs_dir_, tot);
   }
   // Womersley links: the time-independent factor of the profile at the two points
   // a link's velocity is taken at (the Ladd half-way point, and the neighbour the
@@ -382,6 +396,9 @@ StepArgs Solver::args() const {
   a.gen.cpl = g_cpl_.as<int>();
   a.gen.xyz = g_xyz_.as<int>();
   a.gen.wom = g_wom_.as<int>();
+  a.iol_rec = iol_rec_.as<int>();
+  a.iol_dir = iol_dir_.as<uint8_t>();
+  a.iol_n = iol_n_;
   a.gen.gzs = g_gzs_.as<uint32_t>();
   a.gzs_rec = gzs_rec_.as<int>();
   a.gzs_dir = gzs_dir_.as<uint8_t>();
@@ -531,7 +548,7 @@ void Solver::pre_receive(bool macro, int which, bool stress) {
 // Kernels of one step: one for a steady-state step (two with the iolet records
 // beside it), else one per kind of work.
 int Solver::step_launches(bool macro) const {
-  if (direct_ || macro) return 1 + (L_.G > 0 ? 1 : 0) + (gzs_n_ > 0 ? 1 : 0);
+  if (direct_ || macro) return 1 + (L_.G > 0 ? 1 : 0) + (iol_n_ > 0 ? 1 : 0) + (gzs_n_ > 0 ? 1 : 0);
   return 1 + (wk_beside_ && L_.G > L_.kind_start[2] ? 1 : 0);
 }
 

@@ -145,6 +145,8 @@ class Solver {
   DeviceBuffer meta_, run_off_, run_po_, st2ref_;
   DeviceBuffer g_run_;
   DeviceBuffer g_site_, g_wall_, g_iolet_, g_src_, g_q_, g_nrm_, g_io_, g_cpl_, g_xyz_;
+  DeviceBuffer iol_rec_, iol_dir_;   // iolet links
+  int iol_n_ = 0;
   DeviceBuffer g_gzs_, gzs_rec_, gzs_dir_;    // GZS wall links (GZS walls only)
   int gzs_n_ = 0;
   DeviceBuffer g_wom_, wom_amp_;     // Womersley link factors (allocated only with such an iolet)

@@ -14,14 +14,14 @@ namespace {
 
 constexpr int kStepBlock = 128;
 
-// Blocks of a step kernel's grid, in order: `io` blocks of boundary records with
-// iolet links (from record io_first), `gzs` blocks of GZS wall links, then `wall`
+// Blocks of a step kernel's grid, in order: `links` blocks of iolet links, `io`
+// blocks of boundary records with such links (from record io_first), `gzs` blocks of GZS wall links, then `wall`
 // blocks of boundary records without iolet links spread evenly among `bulk` blocks
 // of `tiles` tiles of sites each.
 struct StepTiles {
-  int io, gzs, wall, bulk, tiles, io_first;
+  int links, io, gzs, wall, bulk, tiles, io_first;
   uint32_t wall_share;  // of the last two kinds, 32-bit fraction rounded up
-  int blocks() const { return io + gzs + wall + bulk; }
+  int blocks() const { return links + io + gzs + wall + bulk; }
   // The wall blocks before block b of the last two kinds.
   __device__ __forceinline__ int walls_before(int b) const { return bulk > 0 ? (int)__umulhi((unsigned)b, wall_share) : b; }
 };
@@ -39,7 +39,10 @@ inline StepTiles step_tiles(const StepArgs& a, int which, int resident) {
   StepTiles t{};
   auto blocks = [](int64_t n, int64_t per) { return (int)((n + per - 1) / per); };
   t.io_first = a.gen.G_noiolet;
-  if (which & kLaunchIoletRecords) t.io = blocks(a.gen.G - t.io_first, kStepBlock);
+  if (which & kLaunchIoletRecords) {
+    t.links = blocks(a.iol_n, kStepBlock);
+    t.io = blocks(a.gen.G - t.io_first, kStepBlock);
+  }
   if (which & kLaunchWallRecords) {
     t.gzs = blocks(a.gzs_n, kStepBlock);
     t.wall = blocks(t.io_first, kStepBlock);
