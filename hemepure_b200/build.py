@@ -31,8 +31,8 @@ CU_SOURCES = {
     # the selectors' float arithmetic as the host rounds it
     "extract.cu": ["-fmad=false"],
 }
-CPP_SOURCES = ["xml.cpp", "config.cpp", "layout.cpp", "shard.cpp", "solver.cpp", "extraction.cpp", "batch.cpp", "capi.cpp"]
-HEADERS = ["hb_common.h", "f64_site.cuh", "xml.h", "config.h", "layout.h", "device.h", "solver.h", "extraction.h", "mixed_site.cuh", "batch.h", "batch_dev.h", "shard.h", "setup_pool.h", "step_tiles.cuh"]
+CPP_SOURCES = ["xml.cpp", "config.cpp", "layout.cpp", "shard.cpp", "host_copy.cpp", "solver.cpp", "extraction.cpp", "batch.cpp", "capi.cpp"]
+HEADERS = ["hb_common.h", "f64_site.cuh", "xml.h", "config.h", "layout.h", "device.h", "solver.h", "extraction.h", "mixed_site.cuh", "batch.h", "batch_dev.h", "shard.h", "setup_pool.h", "host_copy.h", "step_tiles.cuh"]
 
 
 def _deps_mtime() -> float:

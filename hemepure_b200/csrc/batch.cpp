@@ -566,23 +566,14 @@ void Batch::get_macro(int slot, double* rho, double* u, double* wss) {
   if (it == members_.end()) throw Error{HB_ERR_ARG, "no such batch member"};
   const BatchMember& m = *it->second;
   if (!m.finished) throw Error{HB_ERR_ARG, "the member has not finished; its fields are filled on its last step"};
-  const int n = m.L.n;
-  std::vector<double> r(n), uu(3 * (size_t)n), w(n);
-  check(cudaMemcpy(r.data(), rho_.as<double>() + m.site_base, n * sizeof(double), cudaMemcpyDeviceToHost), "macro");
-  for (int c = 0; c < 3; c++)
-    check(cudaMemcpy(uu.data() + (size_t)c * n, u_.as<double>() + c * np_ + m.site_base, n * sizeof(double), cudaMemcpyDeviceToHost),
-          "macro");
-  check(cudaMemcpy(w.data(), wss_.as<double>() + m.site_base, n * sizeof(double), cudaMemcpyDeviceToHost), "macro");
-  for (int s = 0; s < n; s++) {
-    const int x = m.L.st2ref[s];
-    if (rho) rho[x] = r[s];
-    if (u) {
-      u[3 * (size_t)x] = uu[s];
-      u[3 * (size_t)x + 1] = uu[(size_t)n + s];
-      u[3 * (size_t)x + 2] = uu[2 * (size_t)n + s];
-    }
-    if (wss) wss[x] = w[s];
-  }
+  auto fetch = [&](const DeviceBuffer& field, int width, double* out) {
+    if (out)
+      host_copy_.field_to_reference(out, field.as<double>() + m.site_base, np_, width, m.L.st2ref.data(), nullptr, m.L.n,
+                                    device_, stream_);
+  };
+  fetch(rho_, 1, rho);
+  fetch(u_, 3, u);
+  fetch(wss_, 1, wss);
 }
 
 }  // namespace hb

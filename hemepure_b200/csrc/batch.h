@@ -119,6 +119,7 @@ class Batch {
   DeviceBuffer f_[2], ghost_[2];
   DeviceBuffer meta_, run_off_;
   DeviceBuffer g_site_, g_run_, g_wall_, g_iolet_, g_src_, g_q_, g_nrm_, g_io_, g_cpl_, g_xyz_, g_lat_;
+  HostCopy host_copy_;
   DeviceBuffer lat_, cos_, iolets_, dens_, lat_status_, macro_list_, macro_count_, io_moments_, iol_list_, iol_link_, rho_, u_, wss_;
   int cur_ = 0;
   int spt_ = 2, bulk_block_ = 256;

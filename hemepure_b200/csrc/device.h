@@ -160,6 +160,9 @@ void launch_select(const SelectArgs& s, uint8_t* mask, int* counts, int* total, 
 // out[k*width + j] = src[j*stride + ref2st[idx[k]]] for k < m (a field in storage order).
 void launch_gather_selected(const double* src, int64_t stride, int width, const int* idx, const int* ref2st, int m,
                             double* out, void* stream);
+// out[st2ref[s]*width + j] = src[j*stride + s] for s < n (a field in storage order to
+// rows in reference order).
+void launch_to_reference(const double* src, int64_t stride, int width, const int* st2ref, int n, double* out, void* stream);
 // out[k*width + j] = aos[idx[k]*width + j] (rows of an array in reference order).
 void launch_gather_rows(const double* aos, int width, const int* idx, int m, double* out, void* stream);
 // Sharded form (shard.cu): out[k] = f[idx[k]] and f[idx[k]] = in[k] over m

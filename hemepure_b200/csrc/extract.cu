@@ -170,6 +170,18 @@ __global__ void __launch_bounds__(kThreads) k_gather_sel(const double* src, int6
   out[t] = src[(int64_t)j * stride + ref2st[idx[k]]];
 }
 
+// out[st2ref[s] * width + j] = src[j * stride + s]: a field in storage order to
+// rows in reference order.  Coalesced reads; the eight consecutive sites of a
+// geometry block's edge are usually neighbours in both orders, so the writes fill
+// 64 bytes or more of a line together.
+__global__ void __launch_bounds__(kThreads) k_to_reference(const double* src, int64_t stride, int width, const int* st2ref,
+                                                           int n, double* out) {
+  const int s = blockIdx.x * kThreads + threadIdx.x;
+  if (s >= n) return;
+  double* o = out + (int64_t)st2ref[s] * width;
+  for (int j = 0; j < width; j++) o[j] = src[(int64_t)j * stride + s];
+}
+
 // out[k * width + j] = aos[idx[k] * width + j]: rows of an AoS array in reference order.
 __global__ void __launch_bounds__(kThreads) k_gather_rows(const double* aos, int width, const int* idx, int m, double* out) {
   const int64_t t = blockIdx.x * (int64_t)kThreads + threadIdx.x;
@@ -199,6 +211,11 @@ void launch_gather_selected(const double* src, int64_t stride, int width, const 
   if (m <= 0) return;
   k_gather_sel<<<blocks_for((int64_t)m * width), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(src, stride, width,
                                                                                                     idx, ref2st, m, out);
+}
+
+void launch_to_reference(const double* src, int64_t stride, int width, const int* st2ref, int n, double* out, void* stream) {
+  if (n <= 0) return;
+  k_to_reference<<<blocks_for(n), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(src, stride, width, st2ref, n, out);
 }
 
 void launch_gather_rows(const double* aos, int width, const int* idx, int m, double* out, void* stream) {

@@ -1,0 +1,110 @@
+// host_copy.cpp -- see host_copy.h.
+#include "host_copy.h"
+
+#include <algorithm>
+#include <cstring>
+#include <string>
+#include <thread>
+#include <vector>
+
+#include "../../include/hemeb200.h"
+#include "device.h"
+#include "hb_common.h"
+#include "setup_pool.h"
+
+namespace hb {
+
+HostCopy::~HostCopy() {
+  for (cudaEvent_t e : done_)
+    if (e) cudaEventDestroy(e);
+  if (pinned_) cudaFreeHost(pinned_);
+}
+
+void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, cudaStream_t stream) {
+  auto check = [](cudaError_t e) {
+    if (e != cudaSuccess) throw Error{HB_ERR_CUDA, std::string("host copy: ") + cudaGetErrorString(e)};
+  };
+  if (bytes == 0) return;
+  bool pieces = bytes > (down ? kDirectDown : kDirectUp);
+  if (pieces && !pinned_) {
+    // Without pinned memory to spare the copy still runs, as a pageable one.
+    if (cudaHostAlloc((void**)&pinned_, kThreads * kPiece, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      pinned_ = nullptr;
+      pieces = false;
+    }
+    for (int k = 0; pieces && k < kThreads; k++)
+      if (!done_[k]) check(cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming));
+  }
+  if (!pieces) {
+    check(cudaMemcpyAsync(down ? host : dev, down ? dev : host, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
+                          stream));
+    check(cudaStreamSynchronize(stream));
+    return;
+  }
+  const size_t count = (bytes + kPiece - 1) / kPiece;
+  const int threads = (int)std::min<size_t>(kThreads, count);
+  cudaError_t err[kThreads];
+  auto work = [&](int k) {
+    unsigned char* piece = pinned_ + (size_t)k * kPiece;
+    cudaError_t e = cudaSetDevice(device);
+    for (size_t p = k; p < count && e == cudaSuccess; p += threads) {
+      unsigned char* h = static_cast<unsigned char*>(host) + p * kPiece;
+      unsigned char* d = static_cast<unsigned char*>(dev) + p * kPiece;
+      const size_t len = std::min(kPiece, bytes - p * kPiece);
+      if (down) {
+        e = cudaMemcpyAsync(piece, d, len, cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaEventRecord(done_[k], stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(done_[k]);
+        if (e == cudaSuccess) std::memcpy(h, piece, len);
+      } else {
+        std::memcpy(piece, h, len);
+        e = cudaMemcpyAsync(d, piece, len, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaEventRecord(done_[k], stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(done_[k]);
+      }
+    }
+    err[k] = e;
+  };
+  std::vector<std::thread> pool;
+  int started = 1;
+  try {
+    for (; started < threads; started++) pool.emplace_back(work, started);
+  } catch (...) {
+    // no more threads to be had: the pieces of the missing ones follow below
+  }
+  work(0);
+  for (auto& t : pool) t.join();
+  for (int k = started; k < threads; k++) work(k);
+  for (int k = 0; k < threads; k++) check(err[k]);
+}
+
+void HostCopy::field_to_reference(double* out, const double* field, int64_t stride, int width, const int* order,
+                                  const int* order_dev, int n, int device, cudaStream_t stream) {
+  auto check = [](cudaError_t e) {
+    if (e != cudaSuccess) throw Error{HB_ERR_CUDA, std::string("field download: ") + cudaGetErrorString(e)};
+  };
+  try {
+    SetupPool tmp(device, stream);
+    double* rows = tmp.get<double>((size_t)n * width);
+    if (!order_dev) {
+      int* o = tmp.get<int>((size_t)n);
+      check(cudaMemcpyAsync(o, order, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, stream));
+      order_dev = o;
+    }
+    launch_to_reference(field, stride, width, order_dev, n, rows, stream);
+    check(cudaGetLastError());
+    to_host(out, rows, (size_t)n * width * sizeof(double), device, stream);
+    return;
+  } catch (const Error& e) {
+    if (e.code != HB_ERR_OOM) throw;
+    cudaGetLastError();
+  }
+  std::vector<double> v((size_t)n);
+  for (int c = 0; c < width; c++) {
+    to_host(v.data(), field + (size_t)c * stride, v.size() * sizeof(double), device, stream);
+    for (int s = 0; s < n; s++) out[(size_t)order[s] * width + c] = v[s];
+  }
+}
+
+}  // namespace hb

@@ -1,0 +1,49 @@
+// host_copy.h -- copies between device memory and the caller's pageable arrays
+// through pinned pieces.
+//
+// A pageable cudaMemcpy runs on one host thread inside the driver, which also
+// takes the page faults of a freshly allocated destination.  Here several
+// threads each own a pinned piece: one piece crosses to the host while the
+// others are copied to or from the caller's array, so the faults and the copies
+// run in parallel with the transfer.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+namespace hb {
+
+class HostCopy {
+ public:
+  HostCopy() = default;
+  HostCopy(const HostCopy&) = delete;
+  HostCopy& operator=(const HostCopy&) = delete;
+  ~HostCopy();
+  // `dst` <- `src` on `stream`; the call returns when the copy is done.
+  void to_host(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream) { run(dst, const_cast<void*>(src), bytes, true, device, stream); }
+  void to_device(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream) { run(const_cast<void*>(src), dst, bytes, false, device, stream); }
+
+  // A field of `width` values a site, [width][stride] in storage order on the
+  // device, to `out` as [n][width] in reference order (`order`: storage index to
+  // reference index; `order_dev` the same on the device, or null).  A kernel
+  // reorders it, so that the host only receives it (density, velocity and
+  // stress of 4M sites: 160 ms with the reordering on the host, 12 ms so); with no device memory left
+  // for the reordered copy the host reorders it.
+  void field_to_reference(double* out, const double* field, int64_t stride, int width, const int* order,
+                          const int* order_dev, int n, int device, cudaStream_t stream);
+
+ private:
+  // 4 MB pinned in all: pinning takes about 0.75 ms a megabyte, once per object.
+  static constexpr int kThreads = 8;
+  static constexpr size_t kPiece = (size_t)512 << 10;
+  // Up to these sizes one pageable copy: a download gains by its destination's page
+  // faults taken in parallel, an upload only by the second copy.
+  static constexpr size_t kDirectDown = (size_t)4 << 20, kDirectUp = (size_t)64 << 20;
+  void run(void* host, void* dev, size_t bytes, bool down, int device, cudaStream_t stream);
+  unsigned char* pinned_ = nullptr;   // kThreads pieces, made at the first large copy
+  cudaEvent_t done_[kThreads] = {};
+};
+
+}  // namespace hb

@@ -11,6 +11,7 @@
 #include "solver.h"
 #include "shard.h"
 #include "extraction.h"
+#include "setup_pool.h"
 
 #include <algorithm>
 #include <cstdio>
@@ -803,28 +804,28 @@ void Solver::set_units(double dt, double dx, const double origin[3]) {
 }
 
 void Solver::get_fs(double* f) {
+  const size_t bytes = (size_t)L_.n * Q * sizeof(double);
   if (mixed()) {
-    DeviceBuffer tmp;
-    tmp.alloc((size_t)L_.n * Q * sizeof(double));
-    to_aos(false, tmp.as<double>());
-    check(cudaMemcpyAsync(f, tmp.p, (size_t)L_.n * Q * sizeof(double), cudaMemcpyDeviceToHost, stream_), "f download");
-    check(cudaStreamSynchronize(stream_), "get_fs");
+    SetupPool tmp(opt_.device, stream_);
+    double* aos = tmp.get<double>((size_t)L_.n * Q);
+    to_aos(false, aos);
+    host_copy_.to_host(f, aos, bytes, opt_.device, stream_);
     return;
   }
   materialise();
   double* aos = f_[1 - cur_].as<double>();  // the spare buffer holds n*19 doubles
   launch_soa_to_aos_f64(f_[cur_].as<double>(), L_.np, st2ref_.as<int>(), L_.n, aos, stream_);
   check(cudaGetLastError(), "soa_to_aos launch");
-  check(cudaMemcpyAsync(f, aos, (size_t)L_.n * Q * sizeof(double), cudaMemcpyDeviceToHost, stream_), "f download");
-  check(cudaStreamSynchronize(stream_), "get_fs");
+  host_copy_.to_host(f, aos, bytes, opt_.device, stream_);
 }
 
 void Solver::set_fs(const double* f) {
+  const size_t bytes = (size_t)L_.n * Q * sizeof(double);
   if (mixed()) {
-    DeviceBuffer tmp;
-    tmp.alloc((size_t)L_.n * Q * sizeof(double));
-    check(cudaMemcpyAsync(tmp.p, f, (size_t)L_.n * Q * sizeof(double), cudaMemcpyHostToDevice, stream_), "f upload");
-    launch_from_aos_mixed(tmp.as<double>(), st2ref_.as<int>(), L_.n, L_.np, opt_.precision, f_[cur_].p, stream_);
+    SetupPool tmp(opt_.device, stream_);
+    double* aos = tmp.get<double>((size_t)L_.n * Q);
+    host_copy_.to_device(aos, f, bytes, opt_.device, stream_);
+    launch_from_aos_mixed(aos, st2ref_.as<int>(), L_.n, L_.np, opt_.precision, f_[cur_].p, stream_);
     check(cudaGetLastError(), "from_aos launch");
     direct_ = true;
     prev_valid_ = false;
@@ -832,7 +833,7 @@ void Solver::set_fs(const double* f) {
     return;
   }
   double* aos = f_[1 - cur_].as<double>();
-  check(cudaMemcpyAsync(aos, f, (size_t)L_.n * Q * sizeof(double), cudaMemcpyHostToDevice, stream_), "f upload");
+  host_copy_.to_device(aos, f, bytes, opt_.device, stream_);
   launch_aos_to_soa_f64(aos, st2ref_.as<int>(), L_.n, f_[cur_].as<double>(), L_.np, stream_);
   check(cudaGetLastError(), "aos_to_soa launch");
   direct_ = true;
@@ -840,25 +841,15 @@ void Solver::set_fs(const double* f) {
   check(cudaStreamSynchronize(stream_), "set_fs");
 }
 
+void Solver::fetch_field(const double* field, int width, double* out) {
+  host_copy_.field_to_reference(out, field, L_.np, width, L_.st2ref.data(), st2ref_.as<int>(), L_.n, opt_.device, stream_);
+}
+
 void Solver::get_macro(double* rho, double* u, double* wss) {
   if (!macro_valid_ || !rho_.p) throw Error{HB_ERR_ARG, "no step has filled the macroscopic caches (pass HB_STEP_MACRO)"};
-  const int n = L_.n;
-  const int64_t np = L_.np;
-  std::vector<double> r(np), uu(3 * np), w(np);
-  check(cudaMemcpyAsync(r.data(), rho_.p, np * sizeof(double), cudaMemcpyDeviceToHost, stream_), "macro download");
-  check(cudaMemcpyAsync(uu.data(), u_.p, 3 * np * sizeof(double), cudaMemcpyDeviceToHost, stream_), "macro download");
-  check(cudaMemcpyAsync(w.data(), wss_.p, np * sizeof(double), cudaMemcpyDeviceToHost, stream_), "macro download");
-  check(cudaStreamSynchronize(stream_), "get_macro");
-  for (int s = 0; s < n; s++) {
-    const int x = L_.st2ref[s];
-    if (rho) rho[x] = r[s];
-    if (u) {
-      u[3 * x] = uu[s];
-      u[3 * x + 1] = uu[np + s];
-      u[3 * x + 2] = uu[2 * np + s];
-    }
-    if (wss) wss[x] = w[s];
-  }
+  if (rho) fetch_field(rho_.as<double>(), 1, rho);
+  if (u) fetch_field(u_.as<double>(), 3, u);
+  if (wss) fetch_field(wss_.as<double>(), 1, wss);
 }
 
 int Solver::stress_len(int field) {
@@ -881,24 +872,15 @@ void Solver::get_stress(int field, double* out) {
   const int k = stress_len(field);
   if (!stress_valid_ || !pi_.p)
     throw Error{HB_ERR_ARG, "no step has filled the stress caches (pass HB_STEP_MACRO | HB_STEP_STRESS)"};
-  const int n = L_.n;
-  const int64_t np = L_.np;
   if (!stress_out_.p) {
-    stress_out_.alloc((size_t)6 * np * sizeof(double));
+    stress_out_.alloc((size_t)6 * L_.np * sizeof(double));
     dev_bytes_ += (int64_t)stress_out_.bytes;
   }
   StepArgs a = args();
   a.pi = pi_.as<double>();
   launch_stress_field(a, field, stress_out_.as<double>(), stream_);
   check(cudaGetLastError(), "stress field launch");
-  std::vector<double> v((size_t)k * np);
-  check(cudaMemcpyAsync(v.data(), stress_out_.p, v.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_),
-        "stress download");
-  check(cudaStreamSynchronize(stream_), "get_stress");
-  for (int s = 0; s < n; s++) {
-    const int64_t x = L_.st2ref[s];
-    for (int c = 0; c < k; c++) out[x * k + c] = v[(size_t)c * np + s];
-  }
+  fetch_field(stress_out_.as<double>(), k, out);
 }
 
 void Solver::moment_sums(double out[4]) {

@@ -10,6 +10,7 @@
 #include "../../include/hemeb200.h"
 #include "config.h"
 #include "device.h"
+#include "host_copy.h"
 #include "layout.h"
 
 namespace hb {
@@ -127,6 +128,7 @@ class Solver {
   void launch_wk3(cudaStream_t st);
   int step_launches(bool macro) const;
   void to_aos(bool use_prev, double* dev_aos);
+  void fetch_field(const double* field, int width, double* out);
 
   LatticeTables t_;
   hb_params p_;
@@ -154,6 +156,7 @@ class Solver {
   DeviceBuffer rho_, u_, wss_;
   DeviceBuffer pi_, stress_out_;  // allocated at the first stress step
   DeviceBuffer sum_scratch_, sum_out_;
+  HostCopy host_copy_;
   int dens_rows_ = 0;
   int row_ = 0;                   // row of the density table used by the current step
   // Pinned, so a step's row upload is a direct asynchronous copy; rows_ev_ marks

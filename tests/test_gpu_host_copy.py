@@ -1,0 +1,39 @@
+"""Fields and distributions large enough to cross to the host in pinned pieces, of a
+size that is no multiple of a piece."""
+
+import numpy as np
+import pytest
+
+from hemepure_b200 import lbm, vessels
+
+pytestmark = pytest.mark.gpu
+
+C = np.array([(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1), (1, 1, 0), (-1, -1, 0),
+              (1, -1, 0), (-1, 1, 0), (1, 0, 1), (-1, 0, -1), (1, 0, -1), (-1, 0, 1), (0, 1, 1), (0, -1, -1), (0, 1, -1),
+              (0, -1, 1)], float)
+
+
+@pytest.mark.parametrize("precision,eps", [("fp64", 2.0 ** -53), ("fp32", 2.0 ** -24)])
+@pytest.mark.parametrize("radius,length", [(6.0, 31), (20.0, 151)])  # u below and above a piece
+def test_fields_arrive_in_reference_order(tmp_path, precision, eps, radius, length):
+    v = vessels.Pipe(radius, length)
+    vessels.voxelise(v, str(tmp_path / "c.gmy"))
+    vessels.write_case_xml(str(tmp_path / "c.xml"), "c.gmy", v, vessels.CaseUnits(tau=0.8), 10, [vessels.VelocityBC(0.01)],
+                           [vessels.PressureBC(1.0)])
+    sim = lbm.LBM(str(tmp_path / "c.xml"), wall="BFL", precision=precision)
+    rng = np.random.default_rng(3)
+    w = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12)
+    f = w * (1.0 + 1e-3 * rng.standard_normal((sim.n, 19)))
+    sim.SetFs(f)
+    got = sim.GetFOld()
+    # FP64 storage is exact; FP32 rounds the deviation from w, at most 5e-3 w.
+    assert np.abs(got - f).max() <= (0.0 if precision == "fp64" else 5e-3 / 3 * eps)
+    sim.step(1, macro=True, stress=True)
+    rho, u, wss = sim.GetPropertyCache()
+    # Sums of 19 rounded values of order 1 and below.
+    assert np.abs(rho - got.sum(1)).max() <= 19 * eps
+    assert np.abs(u - (got @ C) / got.sum(1)[:, None]).max() <= 40 * eps
+    wall = sim.tables()["wall_mask"] != 0
+    assert np.array_equal(wss < 1e300, wall)
+    traction = sim.GetStress("traction")
+    assert np.array_equal((traction != 0).any(1), wall)
