@@ -214,7 +214,8 @@ __global__ void __launch_bounds__(128) k_batch_ghosts(const BatchArgs b) {
       const float nx = (float)I.nrm_f[0], ny = (float)I.nrm_f[1], nz = (float)I.nrm_f[2];
       const float comp = ux * nx + uy * ny + uz * nz;
       const Geq gq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f);
-      v = geq_at(gq, inv(link));
+      const PairF eq = geq_pair(gq, (link - 1) >> 1);
+      v = (link & 1) ? eq.e : eq.o;  // the direction opposite to the link
     }
     b.gout[(int64_t)(link - 1) * G.G + gi] = v;
   }

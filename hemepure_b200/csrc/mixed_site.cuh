@@ -502,19 +502,32 @@ __device__ __forceinline__ void general_site_m(const StepArgs& a, const MixArgs&
   }
 }
 
-// v[i] for an index known at run time only, without an indexed array.
-__device__ __forceinline__ float pick_m(const float* v, int i) {
-  float x = v[1];
+// A link's direction is known at run time only: opposite directions by pairs, as
+// in f64_site.cuh.
+__constant__ float kVelocityF[9][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 1, 0}, {1, -1, 0}, {1, 0, 1}, {1, 0, -1}, {0, 1, 1}, {0, 1, -1}};
+
+struct PairF {
+  float o, e;  // of the odd and of the even direction
+};
+
+__device__ __forceinline__ PairF pick_pair_m(const float* v, int p) {
+  PairF x{v[1], v[2]};
 #pragma unroll
-  for (int k = 2; k < Q; k++) x = k == i ? v[k] : x;
+  for (int k = 1; k < 9; k++) {
+    x.o = k == p ? v[2 * k + 1] : x.o;
+    x.e = k == p ? v[2 * k + 2] : x.e;
+  }
   return x;
 }
 
-// Equilibrium of a direction known at run time only.
-__device__ __forceinline__ float geq_at(const Geq& c, int i) {
-  const float w = i < 7 ? wf(1) : wf(7);
-  const float e = (float)cx(i) * c.mx + (float)cy(i) * c.my + (float)cz(i) * c.mz;
-  return vfma(w, e, vfma(w * c.nh * e, e, w * c.t1));
+__device__ __forceinline__ float pair_weight_m(int p) { return p < 3 ? wf(1) : wf(7); }
+
+// Equilibria of the pair (Geq::pair).
+__device__ __forceinline__ PairF geq_pair(const Geq& c, int p) {
+  const float w = pair_weight_m(p);
+  const float e = vfma(kVelocityF[p][0], c.mx, vfma(kVelocityF[p][1], c.my, vmul(kVelocityF[p][2], c.mz)));
+  const float even = vfma(vmul(vmul(w, c.nh), e), e, vmul(w, c.t1));
+  return PairF{vfma(w, e, even), vfma(-w, e, even)};
 }
 
 // The virtual-node value of entry k of the GZS link list, one thread per link
@@ -548,18 +561,25 @@ __device__ __forceinline__ void gzs_link_m(const StepArgs& a, const MixArgs& m, 
   const Moments mo(g);
   const Geq geq(mo, kScale);
   const float rho = kScale + mo.D;
-  float fi = pick_m(g, i) - geq_at(geq, i), fd = pick_m(g, d) - geq_at(geq, d);
+  const int p = (d - 1) >> 1;
+  const bool odd = d & 1;  // link d is the pair's odd direction
+  PairF n = pick_pair_m(g, p);
+  {
+    const PairF eq = geq_pair(geq, p);
+    n.o -= eq.o;
+    n.e -= eq.e;
+  }
   const float fac = 1.0f - 1.0f / q;
   float mw0 = mo.mx * fac, mw1 = mo.my * fac, mw2 = mo.mz * fac;
   if (extrapolate) {
     const Moments mn(gn);
-    const Geq geqn(mn, kScale);
     const float k2 = (1.0f - q) * rho * (q - 1.0f) / (q + 1.0f) / (kScale + mn.D);
     mw0 = q * mw0 + k2 * mn.mx;
     mw1 = q * mw1 + k2 * mn.my;
     mw2 = q * mw2 + k2 * mn.mz;
-    fi = q * fi + (1.0f - q) * (pick_m(gn, i) - geq_at(geqn, i));
-    fd = q * fd + (1.0f - q) * (pick_m(gn, d) - geq_at(geqn, d));
+    const PairF x = pick_pair_m(gn, p), eq = geq_pair(Geq(mn, kScale), p);
+    n.o = q * n.o + (1.0f - q) * (x.o - eq.o);
+    n.e = q * n.e + (1.0f - q) * (x.e - eq.e);
   } else if (q < 0.75f) {  // behind the site: a velocity iolet
     const int io = __ldg(G.io + gi);
     const double p3[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
@@ -573,10 +593,15 @@ __device__ __forceinline__ void gzs_link_m(const StepArgs& a, const MixArgs& m, 
     mw1 = q * mw1 + k2 * nv[1];
     mw2 = q * mw2 + k2 * nv[2];
   }
-  const float gw_i = geq_at(Geq(Moments(mo.D, mw0, mw1, mw2), kScale), i) + fi;
+  const PairF eqw = geq_pair(Geq(Moments(mo.D, mw0, mw1, mw2), kScale), p);
+  const float fi = odd ? n.e : n.o, gw_i = (odd ? eqw.e : eqw.o) + fi;
   float v;
-  if (K == kTRT) v = gw_i + 0.5f * (float)a.omega * (fi + fd) + 0.5f * (float)a.omega_minus * (fi - fd);
-  else v = gw_i + fi * (float)a.omega;
+  if (K == kTRT) {
+    const float sym = 0.5f * (float)a.omega * (n.o + n.e), asym = 0.5f * (float)a.omega_minus * (n.o - n.e);
+    v = odd ? gw_i + sym - asym : gw_i + sym + asym;
+  } else {
+    v = gw_i + fi * (float)a.omega;
+  }
   Store<S>::st(static_cast<S*>(m.fout) + (int64_t)d * a.np + s, v);
 }
 
@@ -607,20 +632,21 @@ __device__ __forceinline__ void iolet_link_m(const StepArgs& a, const MixArgs& m
     for (int i = 0; i < Q; i++) g[i] = Store<S>::ld(p + (int64_t)i * a.np);
   }
   const Moments mo(g);
-  const int io = __ldg(G.io + gi), i = (d & 1) ? d + 1 : d - 1;
+  const int io = __ldg(G.io + gi), p = (d - 1) >> 1;
+  const bool odd = d & 1;
   const IoletDev& I = a.iolets[io];
   float v;
   if (is_velocity_iolet(I.kind)) {
     float neq[Q], tau, om, w[3];
     non_equilibrium(Geq(mo, kScale), g, neq);
     site_rate<S, K>(a, neq, s, tau, om);
-    const float nd = pick_m(neq, d);
-    float post;
+    const PairF x = pick_pair_m(g, p), n = pick_pair_m(neq, p);
+    float post = odd ? x.o : x.e;
     if (K == kTRT) {
-      const float ni = pick_m(neq, i);
-      post = vfma(0.5f * (float)a.omega_minus, vsub(nd, ni), vfma(0.5f * om, vadd(nd, ni), pick_m(g, d)));
+      post = vfma(0.5f * om, vadd(n.o, n.e), post);
+      post = vfma((odd ? 0.5f : -0.5f) * (float)a.omega_minus, vsub(n.o, n.e), post);
     } else {
-      post = vfma(om, nd, pick_m(g, d));
+      post = vfma(om, odd ? n.o : n.e, post);
     }
     const double pos[3] = {(double)__ldg(G.xyz + gi), (double)__ldg(G.xyz + G.G + gi), (double)__ldg(G.xyz + 2 * G.G + gi)};
     if (!link_velocity_f(a, I, io, gi, d, true, pos, w)) {
@@ -628,7 +654,8 @@ __device__ __forceinline__ void iolet_link_m(const StepArgs& a, const MixArgs& m
       w[0] = w[1] = w[2] = 0.0f;
     }
     const float rho = 1.0f + mo.D * (1.0f / kScale);
-    const float corr = 2.0f * (d < 7 ? wf(1) : wf(7)) * rho * (w[0] * cx(d) + w[1] * cy(d) + w[2] * cz(d)) * 3.0f;
+    const float wc = w[0] * kVelocityF[p][0] + w[1] * kVelocityF[p][1] + w[2] * kVelocityF[p][2];
+    const float corr = 2.0f * pair_weight_m(p) * rho * (odd ? wc : -wc) * 3.0f;
     v = post * (1.0f / kScale) - corr;
   } else {
     const float r = kScale + mo.D;
@@ -638,7 +665,8 @@ __device__ __forceinline__ void iolet_link_m(const StepArgs& a, const MixArgs& m
     const float rbf = (float)rb;
     const float nx = (float)I.nrm_f[0], ny = (float)I.nrm_f[1], nz = (float)I.nrm_f[2];
     const float comp = ux * nx + uy * ny + uz * nz;
-    v = geq_at(Geq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f), i);
+    const PairF eq = geq_pair(Geq(Moments(drb, nx * comp * rbf, ny * comp * rbf, nz * comp * rbf), 1.0f), p);
+    v = odd ? eq.e : eq.o;  // the direction opposite to the link
   }
   m.gout[(int64_t)(d - 1) * G.G + gi] = v;
 }
