@@ -324,13 +324,13 @@ def main():
     if os.path.exists(tp):
         with open(tp) as fh:
             tj = json.load(fh)
-        if tj.get("workload") == args.workload and tj.get("kernel") == "k_bulk":
+        if tj.get("workload") == args.workload and tj.get("kernel") == "k_step":
             traffic = tj.get("bytes_per_launch")
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "kernel": "k_bulk (plain bulk sites)", "peak_kind": peak_kind,
+                "traffic": traffic, "kernel": "k_step (plain bulk tiles alone)", "peak_kind": peak_kind,
                 "algorithmic_bytes_per_launch": bytes_per_site * lay["bulk_sites"], "launch_ms": bulk_launch_ms,
                 "boundary_kernel_alone_ms": g_ms / prof_steps,
-                "step_launches": {"kernels": "k_bulk + k_general_walls + k_general side by side", "ms": step_launch_ms,
+                "step_launches": {"kernels": "k_step (boundary records and plain bulk tiles in one launch)", "ms": step_launch_ms,
                                   "achieved": bytes_per_site * n_sites / (step_launch_ms * 1e-3) / 1e9},
                 "whole_step_frac": (bytes_per_site * n_sites / (ms / args.steps * 1e-3) / 1e9) / peak}
 

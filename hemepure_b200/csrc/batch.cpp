@@ -96,9 +96,8 @@ Batch::Batch(int64_t site_capacity, int64_t general_capacity, int max_lattices, 
   check(cudaSetDevice(device_), "cudaSetDevice");
   cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device_);
   check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-  // The latency-bound boundary kernel runs on the side stream at the highest
-  // priority, so its blocks are dispatched ahead of the bulk kernel's queued ones
-  // (4M-site pipe: FP32 step 29.3k -> 30.3k MLUPS; FP64 unchanged).
+  // The latency-bound boundary tiles run on the side stream at the highest
+  // priority, so their blocks are dispatched ahead of the bulk tiles' queued ones.
   int prio_lo = 0, prio_hi = 0;
   check(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi), "cudaDeviceGetStreamPriorityRange");
   check(cudaStreamCreateWithPriority(&side_, cudaStreamNonBlocking, prio_hi), "cudaStreamCreate");

@@ -34,17 +34,16 @@ constexpr int kStepBlocksPerSM = 4;
 // One steady-state time step (gathering, no outputs) in one launch: the grid's
 // blocks of kStepBlock threads take iolet links, boundary records with such links,
 // GZS wall links, boundary records without iolet links and plain bulk sites
-// (StepTiles).
-// The bulk blocks are bound by HBM bandwidth and the boundary blocks by latency,
+// (StepTiles).  The bulk blocks are bound by HBM bandwidth and the boundary blocks by latency,
 // so the wall-record blocks are spread evenly among the bulk blocks instead of
 // running ahead of them, and the long iolet and link blocks come first.  The
 // kernel is launched with programmatic dependent launch: its blocks load their
 // constant tables while the previous step drains and wait for it before reading
 // distributions.  Three kernels on three streams, forked and joined by events,
 // before: 13k-site pipe 11.6 -> 7.7 us a step, 497k-site LES stenosis 44.0 -> 34.6,
-// 594k-site GZS bifurcation 105 -> 96, 4M-site pipe 213.5 -> 207.9.  Four blocks of 128 (128 registers, what the BFL gather
-// of the wall records takes) against five (102): 4M-site pipe 214 / 216 us, LES
-// stenosis 36 / 40.
+// 594k-site GZS bifurcation 105 -> 96, 4M-site pipe 213.5 -> 207.9.  Four blocks of
+// 128 (128 registers, what the BFL gather of the wall records takes) against five
+// (102): 4M-site pipe 208 / 216 us, LES stenosis 36 / 40.
 template <int K, int WALL>
 __global__ void __launch_bounds__(kStepBlock, kStepBlocksPerSM) k_step(const StepArgs a, const StepTiles t) {
   int b = blockIdx.x;

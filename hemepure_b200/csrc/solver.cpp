@@ -4,7 +4,7 @@
 //   RequestComms   Windkessel DoComms on the device (k_wk3_begin), cosine
 //                  densities from the host table (InOutLetCosine::GetDensity with
 //                  the 0-indexed step, BoundaryValues.cc:211-214)
-//   PreReceive     k_bulk over plain bulk sites, k_general over the rest
+//   PreReceive     every site: one kernel in a steady-state step (k_step)
 //   PostReceive    nothing: the BFL post-step is applied when the next step
 //                  gathers (kernels_f64.cu)
 //   EndIteration   swap the two buffers, time step + 1
@@ -629,8 +629,8 @@ int Solver::profile(int64_t nsteps, double ms[3]) {
   cudaEvent_t e[3];
   for (auto& x : e) check(cudaEventCreate(&x), "cudaEventCreate");
   int rc = HB_OK;
-  // Pass 0: the launches hb_step issues; pass 1: the bulk and boundary kernels
-  // one after the other.
+  // Pass 0: the launches hb_step issues; pass 1: the bulk sites and the boundary
+  // records one after the other.
   for (int pass = 0; pass < 2; pass++) {
     for (int64_t j = 0; j < nsteps; j++) {
       {

@@ -473,7 +473,7 @@ class LBM:
 
     def profile_steps(self, n: int):
         """Advance 2n steps timing the launches: (step launch ms over the first n
-        steps as `step` runs them, plain-bulk kernel ms and boundary kernel ms
+        steps as `step` runs them, plain bulk sites' ms and boundary records' ms
         over the next n steps run one kernel after the other)."""
         ms = np.zeros(3)
         self._check(library().hb_profile_steps(self._h, int(n), _p(ms)))

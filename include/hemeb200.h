@@ -482,9 +482,9 @@ int hb_last_step_timing(const hb_handle* h, double* ms, int64_t* launches);
 int hb_setup_timing(const hb_handle* h, double ms[4]);
 /* Advance 2 x `n_steps` steps with CUDA events around the launches (for
  * measurement only).  The first n_steps run as hb_step runs them and ms[0]
- * sums their collide-and-stream launch (one fused kernel, or the bulk and
- * boundary kernels side by side); the next n_steps run the plain-bulk kernel
- * and then the boundary kernel, and ms[1] and ms[2] sum those. */
+ * sums their collide-and-stream launch (plain bulk sites and boundary records
+ * together); the next n_steps run the plain bulk sites and then the boundary
+ * records, and ms[1] and ms[2] sum those. */
 int hb_profile_steps(hb_handle* h, int64_t n_steps, double ms[3]);
 /* Bytes of device memory held by the handle. */
 int hb_device_bytes(const hb_handle* h, int64_t* bytes);
