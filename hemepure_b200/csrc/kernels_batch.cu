@@ -189,9 +189,12 @@ __global__ void __launch_bounds__(128) k_batch_ghosts(const BatchArgs b) {
     const int l = __ldg(b.g_lat + gi);
     if (l < 0) continue;
     const BatchLatDev& d = b.lat[l];
-    if (!d.active || d.macro) continue;
+    if (!d.active) continue;
     const int io = __ldg(G.io + gi);
     const IoletDev& I = b.base.iolets[32 * (int64_t)l + io];
+    // A lattice in its last step needs no ghosts any more, but its links' points are
+    // checked against their iolet's radius: with one step to run it is the only check.
+    if (d.macro && I.kind != kParabolic) continue;
     const float rho = b.io_moments[gi];
     float v;
     if (I.kind == kParabolic) {
@@ -203,6 +206,7 @@ __global__ void __launch_bounds__(128) k_batch_ghosts(const BatchArgs b) {
         atomicOr(b.lat_status + l, kStatusIoletRadius);
         w[0] = w[1] = w[2] = 0.0f;
       }
+      if (d.macro) continue;
       const float corr = 2.0f * wf(link) * rho * (w[0] * cx(link) + w[1] * cy(link) + w[2] * cz(link)) * 3.0f;
       v = Store<S>::ld(static_cast<const S*>(b.fout) + (int64_t)link * b.base.np + s) * (1.0f / Store<S>::kScale) - corr;
     } else {

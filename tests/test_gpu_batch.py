@@ -151,3 +151,24 @@ def test_every_launch_shape_gives_the_same_result(mix, tuning):
             fin = a < 1e300
             assert np.array_equal(fin, m < 1e300)
             assert np.max(np.abs(a[fin] - m[fin])) <= 1e-5 * np.max(np.abs(a[fin])), (name, tuning)
+
+
+@pytest.mark.parametrize("form", ["persistent", "split"])
+@pytest.mark.parametrize("steps", [1, 2, 64])
+def test_links_outside_their_iolet_are_reported(tmp_path, form, steps):
+    """A velocity inlet whose radius is smaller than the vessel's: the member comes
+    back with a status, as the single lattice does, also when its only step is its
+    last."""
+    v = vessels.Pipe(6, 20)
+    xml = str(tmp_path / "c.xml")
+    vessels.voxelise(v, str(tmp_path / "c.gmy"))
+    vessels.write_case_xml(xml, "c.gmy", v, vessels.CaseUnits(tau=0.8), 100, [vessels.VelocityBC(0.01, radius=4.0)],
+                           [vessels.PressureBC(1.0)])
+    with pytest.raises(lbm.HemeLBError) as e:
+        lbm.LBM(xml, precision="fp32").step(steps)
+    b = lbm.Batch(20_000, 20_000, 2)
+    b.set_tuning(1, 128, form)
+    slot = b.add_xml(xml, "LBGK", "SBB", steps)
+    while not b.run(64):
+        pass
+    assert b.info(slot)[2] != 0, e.value
