@@ -14,6 +14,30 @@
 
 namespace hb {
 
+namespace {
+
+// The device of a transfer, current in the calling thread while it runs: its kernel
+// and events need it, and a thread that only reads fields may have another.
+class OnDevice {
+ public:
+  explicit OnDevice(int device) {
+    if (cudaGetDevice(&before_) != cudaSuccess) before_ = device;
+    if (before_ != device) cudaSetDevice(device);
+    changed_ = before_ != device;
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+  ~OnDevice() {
+    if (changed_) cudaSetDevice(before_);
+  }
+
+ private:
+  int before_ = 0;
+  bool changed_ = false;
+};
+
+}  // namespace
+
 HostCopy::~HostCopy() {
   for (cudaEvent_t e : done_)
     if (e) cudaEventDestroy(e);
@@ -25,6 +49,7 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
     if (e != cudaSuccess) throw Error{HB_ERR_CUDA, std::string("host copy: ") + cudaGetErrorString(e)};
   };
   if (bytes == 0) return;
+  const OnDevice on(device);
   bool pieces = bytes > (down ? kDirectDown : kDirectUp);
   if (pieces && !pinned_) {
     // Without pinned memory to spare the copy still runs, as a pageable one.
@@ -84,6 +109,7 @@ void HostCopy::field_to_reference(double* out, const double* field, int64_t stri
   auto check = [](cudaError_t e) {
     if (e != cudaSuccess) throw Error{HB_ERR_CUDA, std::string("field download: ") + cudaGetErrorString(e)};
   };
+  const OnDevice on(device);
   try {
     SetupPool tmp(device, stream);
     double* rows = tmp.get<double>((size_t)n * width);

@@ -1,0 +1,145 @@
+// Drives host_copy.cpp on the CPU: the CUDA runtime calls it makes are implemented
+// here on host memory, with the rules that matter to it (a stream, an event and a
+// kernel launch belong to a device; which device is current is a thread's own).
+// Usage: host_copy_main SCENARIO; exits 0 when the scenario's checks hold.
+#include <cuda_runtime.h>
+
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <mutex>
+#include <string>
+#include <thread>
+#include <vector>
+
+#include "../../include/hemeb200.h"
+#include "../../hemepure_b200/csrc/device.h"
+#include "../../hemepure_b200/csrc/host_copy.h"
+#include "../../hemepure_b200/csrc/setup_pool.h"
+
+namespace {
+
+struct FakeStream { int device; };
+struct FakeEvent { int device; };
+thread_local int current = 0;
+thread_local cudaError_t last = cudaSuccess;
+std::mutex mu;
+std::map<void*, size_t> pool_blocks;
+
+cudaError_t note(cudaError_t e) {
+  if (e != cudaSuccess) last = e;
+  return e;
+}
+FakeStream* of(cudaStream_t s) { return reinterpret_cast<FakeStream*>(s); }
+FakeEvent* of(cudaEvent_t e) { return reinterpret_cast<FakeEvent*>(e); }
+
+void require(bool ok, const char* what) {
+  if (ok) return;
+  std::fprintf(stderr, "failed: %s\n", what);
+  std::exit(1);
+}
+
+}  // namespace
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { *d = current; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
+cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
+const char* cudaGetErrorString(cudaError_t) { return "simulated error"; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  *e = reinterpret_cast<cudaEvent_t>(new FakeEvent{current});
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) { delete of(e); return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  return note(e && of(e)->device == of(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle);
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { return note(e ? cudaSuccess : cudaErrorInvalidResourceHandle); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) {
+  *p = std::malloc(n);
+  std::lock_guard<std::mutex> lock(mu);
+  pool_blocks[*p] = n;
+  return cudaSuccess;
+}
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) {
+  std::lock_guard<std::mutex> lock(mu);
+  pool_blocks.erase(p);
+  std::free(p);
+  return cudaSuccess;
+}
+}
+
+namespace hb {
+cudaMemPool_t setup_pool(int, bool) { return nullptr; }
+// The kernel's work, refused where a launch would be: a stream of a device that is not current.
+void launch_to_reference(const double* src, int64_t stride, int width, const int* st2ref, int n, double* out, void* stream) {
+  if (static_cast<FakeStream*>(stream)->device != current) {
+    last = cudaErrorInvalidResourceHandle;
+    return;
+  }
+  for (int s = 0; s < n; s++)
+    for (int j = 0; j < width; j++) out[(int64_t)st2ref[s] * width + j] = src[(int64_t)j * stride + s];
+}
+}  // namespace hb
+
+namespace {
+
+// A field of `n` sites, `width` values each, in storage order, and its reference order.
+struct Field {
+  int n, width;
+  std::vector<double> storage, expect, out;
+  std::vector<int> order;
+  Field(int n_, int width_) : n(n_), width(width_), storage((size_t)n * width), expect(storage.size()), out(storage.size()), order(n) {
+    for (int s = 0; s < n; s++) order[s] = (int)(((int64_t)s * 7919 + 13) % n);  // 7919 is prime: a permutation of n that it does not divide
+    for (int j = 0; j < width; j++)
+      for (int s = 0; s < n; s++) {
+        storage[(size_t)j * n + s] = 10.0 * s + j;
+        expect[(size_t)order[s] * width + j] = 10.0 * s + j;
+      }
+  }
+  void fetch(hb::HostCopy& c, int device, FakeStream& st) {
+    std::fill(out.begin(), out.end(), -1.0);
+    c.field_to_reference(out.data(), storage.data(), n, width, order.data(), order.data(), n, device, reinterpret_cast<cudaStream_t>(&st));
+  }
+};
+
+// A thread whose current device is 0 reads the fields of a handle on device 1.
+void other_device() {
+  for (int n : {1000, 400001}) {
+    hb::HostCopy copy;
+    FakeStream st{1};
+    Field f(n, 3);
+    current = 0;
+    f.fetch(copy, 1, st);
+    require(f.out == f.expect, "field of another device");
+    require(current == 0, "the caller's device is left as it was");
+    std::vector<double> up(f.n * 24), back(up.size());
+    for (size_t k = 0; k < up.size(); k++) up[k] = (double)k;
+    copy.to_device(back.data(), up.data(), up.size() * sizeof(double), 1, reinterpret_cast<cudaStream_t>(&st));
+    require(up == back, "upload to another device");
+    require(current == 0, "the caller's device is left as it was by an upload");
+  }
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::string s = argc > 1 ? argv[1] : "";
+  try {
+    if (s == "other_device") other_device();
+    else return 2;
+  } catch (const hb::Error& e) {
+    std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());
+    return 1;
+  }
+  return 0;
+}
