@@ -51,16 +51,18 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
   if (bytes == 0) return;
   const OnDevice on(device);
   bool pieces = bytes > (down ? kDirectDown : kDirectUp);
-  if (pieces && !pinned_) {
-    // Without pinned memory to spare the copy still runs, as a pageable one.
-    if (cudaHostAlloc((void**)&pinned_, kThreads * kPiece, cudaHostAllocDefault) != cudaSuccess) {
+  // Without pinned memory or events to spare the copy still runs, as a pageable one.
+  if (pieces && !pinned_ && cudaHostAlloc((void**)&pinned_, kThreads * kPiece, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    pinned_ = nullptr;
+    pieces = false;
+  }
+  for (int k = 0; pieces && k < kThreads; k++)
+    if (!done_[k] && cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
-      pinned_ = nullptr;
+      done_[k] = nullptr;
       pieces = false;
     }
-    for (int k = 0; pieces && k < kThreads; k++)
-      if (!done_[k]) check(cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming));
-  }
   if (!pieces) {
     check(cudaMemcpyAsync(down ? host : dev, down ? dev : host, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
                           stream));

@@ -27,6 +27,7 @@ thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
 std::mutex mu;
 std::map<void*, size_t> pool_blocks;
+int events_until_failure = -1;  // calls that still succeed before one fails; -1: none fails
 
 cudaError_t note(cudaError_t e) {
   if (e != cudaSuccess) last = e;
@@ -54,6 +55,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  if (events_until_failure >= 0 && events_until_failure-- == 0) return note(cudaErrorMemoryAllocation);
   *e = reinterpret_cast<cudaEvent_t>(new FakeEvent{current});
   return cudaSuccess;
 }
@@ -130,12 +132,28 @@ void other_device() {
   }
 }
 
+// An event that cannot be made costs speed at most, then and later.
+void event_failure() {
+  for (int good : {0, 3, 7}) {
+    hb::HostCopy copy;
+    FakeStream st{0};
+    Field f(400001, 3);
+    events_until_failure = good;
+    for (int pass = 0; pass < 3; pass++) {
+      f.fetch(copy, 0, st);
+      require(f.out == f.expect, "field after a failed event");
+    }
+    events_until_failure = -1;
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   try {
     if (s == "other_device") other_device();
+    else if (s == "event_failure") event_failure();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());
