@@ -51,6 +51,13 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
   if (bytes == 0) return;
   const OnDevice on(device);
   bool pieces = bytes > (down ? kDirectDown : kDirectUp);
+  if (pieces) {
+    // Memory that CUDA knows (the caller pinned or allocated it through CUDA) needs no
+    // pieces, and device memory must meet the copy's own check, not the host's memcpy.
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) cudaGetLastError();
+    else if (attr.type != cudaMemoryTypeUnregistered) pieces = false;
+  }
   // Without pinned memory or events to spare the copy still runs, as a pageable one.
   if (pieces && !pinned_ && cudaHostAlloc((void**)&pinned_, kThreads * kPiece, cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();

@@ -27,6 +27,9 @@ thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
 std::mutex mu;
 std::map<void*, size_t> pool_blocks;
+void* own_memory = nullptr;  // a caller's buffer that CUDA knows, of this type
+cudaMemoryType own_type = cudaMemoryTypeUnregistered;
+std::atomic<int> copies{0};     // cudaMemcpyAsync calls
 int events_until_failure = -1;  // calls that still succeed before one fails; -1: none fails
 
 cudaError_t note(cudaError_t e) {
@@ -49,7 +52,15 @@ cudaError_t cudaGetDevice(int* d) { *d = current; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t) { return "simulated error"; }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+  std::memset(a, 0, sizeof(*a));
+  a->type = p == own_memory ? own_type : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t) {
+  copies++;
+  if (own_type == cudaMemoryTypeDevice && own_memory && own_memory == (kind == cudaMemcpyDeviceToHost ? d : s))
+    return note(cudaErrorInvalidValue);
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
@@ -147,6 +158,36 @@ void event_failure() {
   }
 }
 
+// A caller's pinned or managed array takes one copy of its own, and device memory
+// given for an array is refused by that copy instead of being written by the host.
+void own_buffers() {
+  const size_t n = (size_t)12 << 20;
+  std::vector<double> a(n), b(n);
+  for (size_t k = 0; k < n; k++) a[k] = (double)k;
+  FakeStream st{0};
+  auto stream = reinterpret_cast<cudaStream_t>(&st);
+  for (cudaMemoryType type : {cudaMemoryTypeHost, cudaMemoryTypeManaged, cudaMemoryTypeDevice}) {
+    for (bool down : {true, false}) {
+      hb::HostCopy copy;
+      std::fill(b.begin(), b.end(), -1.0);
+      own_type = type;
+      own_memory = down ? b.data() : a.data();
+      copies = 0;
+      int code = 0;
+      try {
+        if (down) copy.to_host(b.data(), a.data(), n * sizeof(double), 0, stream);
+        else copy.to_device(b.data(), a.data(), n * sizeof(double), 0, stream);
+      } catch (const hb::Error& e) {
+        code = e.code;
+      }
+      own_memory = nullptr;
+      require(copies == 1, "one copy");
+      if (type == cudaMemoryTypeDevice) require(code == HB_ERR_CUDA && b[0] == -1.0 && b[n - 1] == -1.0, "device memory is refused");
+      else require(code == 0 && a == b, "copied");
+    }
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -154,6 +195,7 @@ int main(int argc, char** argv) {
   try {
     if (s == "other_device") other_device();
     else if (s == "event_failure") event_failure();
+    else if (s == "own_buffers") own_buffers();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());

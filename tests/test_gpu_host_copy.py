@@ -1,8 +1,11 @@
 """Fields and distributions large enough to cross to the host in pinned pieces, of a
 size that is no multiple of a piece."""
 
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
 from hemepure_b200 import lbm, vessels
 
@@ -37,3 +40,15 @@ def test_fields_arrive_in_reference_order(tmp_path, precision, eps, radius, leng
     assert np.array_equal(wss < 1e300, wall)
     traction = sim.GetStress("traction")
     assert np.array_equal((traction != 0).any(1), wall)
+
+
+def test_callers_pinned_array(tmp_path):
+    v = vessels.Pipe(20.0, 151)
+    vessels.voxelise(v, str(tmp_path / "c.gmy"))
+    vessels.write_case_xml(str(tmp_path / "c.xml"), "c.gmy", v, vessels.CaseUnits(tau=0.8), 10, [vessels.VelocityBC(0.01)],
+                           [vessels.PressureBC(1.0)])
+    sim = lbm.LBM(str(tmp_path / "c.xml"), wall="BFL")
+    sim.step(3)
+    pinned = torch.zeros((sim.n, 19), dtype=torch.float64, pin_memory=True)
+    assert lbm.library().hb_get_fs(sim._h, ctypes.cast(pinned.data_ptr(), ctypes.POINTER(ctypes.c_double))) == 0
+    assert np.array_equal(pinned.numpy(), sim.GetFOld())
