@@ -1,8 +1,12 @@
 // host_copy.cpp -- see host_copy.h.
 #include "host_copy.h"
 
+#include <sys/mman.h>
+
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -38,11 +42,99 @@ class OnDevice {
 
 }  // namespace
 
-HostCopy::~HostCopy() {
-  for (cudaEvent_t e : done_)
-    if (e) cudaEventDestroy(e);
-  if (pinned_) cudaFreeHost(pinned_);
-}
+// The process's sets of pinned pieces.  The memory is the library's own, registered
+// with CUDA: should the device's context have been replaced since, it is still there
+// and is registered again.
+class HostCopy::Sets {
+ public:
+  static Sets& get() {
+    static Sets* s = new Sets;  // handles may be destroyed after the statics are
+    return *s;
+  }
+  // A set for one transfer; null without memory to pin, or with kSets lent already.
+  unsigned char* take() {
+    unsigned char* p = nullptr;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      if (!free_.empty()) {
+        p = free_.back();
+        free_.pop_back();
+      } else if (made_ == kSets) {
+        return nullptr;
+      } else {
+        made_++;
+      }
+    }
+    if (!p) {
+      p = static_cast<unsigned char*>(std::aligned_alloc(kHugePage, kBytes));
+      if (p) madvise(p, kBytes, MADV_HUGEPAGE);  // two pages to pin instead of a thousand
+    }
+    if (p && !pinned(p) && cudaHostRegister(p, kBytes, cudaHostRegisterPortable) != cudaSuccess) {
+      cudaGetLastError();
+      std::free(p);
+      p = nullptr;
+    }
+    if (!p) {
+      std::lock_guard<std::mutex> lock(mu_);
+      made_--;
+    }
+    return p;
+  }
+  void give(unsigned char* p) {
+    std::lock_guard<std::mutex> lock(mu_);
+    free_.push_back(p);
+  }
+  void enter() {
+    std::lock_guard<std::mutex> lock(mu_);
+    users_++;
+  }
+  void leave() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (--users_ > 0) return;
+    for (; free_.size() > 1; free_.pop_back(), made_--) {
+      if (cudaHostUnregister(free_.back()) != cudaSuccess) cudaGetLastError();
+      std::free(free_.back());
+    }
+  }
+
+ private:
+  static constexpr size_t kHugePage = (size_t)2 << 20, kBytes = kThreads * kPiece;
+  static_assert(kBytes % kHugePage == 0, "aligned_alloc takes a multiple of the alignment");
+  static bool pinned(const void* p) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, p) == cudaSuccess) return attr.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+  }
+  std::mutex mu_;
+  std::vector<unsigned char*> free_;
+  int made_ = 0, users_ = 0;
+};
+
+// A set and the events of one transfer.
+struct HostCopy::Borrowed {
+  unsigned char* set = nullptr;
+  cudaEvent_t done[kThreads] = {};
+  bool take() {
+    set = Sets::get().take();
+    if (!set) return false;
+    for (cudaEvent_t& e : done)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        e = nullptr;
+        return false;
+      }
+    return true;
+  }
+  ~Borrowed() {
+    for (cudaEvent_t e : done)
+      if (e) cudaEventDestroy(e);
+    if (set) Sets::get().give(set);
+  }
+};
+
+HostCopy::HostCopy() { Sets::get().enter(); }
+HostCopy::~HostCopy() { Sets::get().leave(); }
 
 void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, cudaStream_t stream) {
   auto check = [](cudaError_t e) {
@@ -59,17 +151,8 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
     else if (attr.type != cudaMemoryTypeUnregistered) pieces = false;
   }
   // Without pinned memory or events to spare the copy still runs, as a pageable one.
-  if (pieces && !pinned_ && cudaHostAlloc((void**)&pinned_, kThreads * kPiece, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    pinned_ = nullptr;
-    pieces = false;
-  }
-  for (int k = 0; pieces && k < kThreads; k++)
-    if (!done_[k] && cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      done_[k] = nullptr;
-      pieces = false;
-    }
+  Borrowed b;
+  pieces = pieces && b.take();
   if (!pieces) {
     check(cudaMemcpyAsync(down ? host : dev, down ? dev : host, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
                           stream));
@@ -80,7 +163,7 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
   const int threads = (int)std::min<size_t>(kThreads, count);
   cudaError_t err[kThreads];
   auto work = [&](int k) {
-    unsigned char* piece = pinned_ + (size_t)k * kPiece;
+    unsigned char* piece = b.set + (size_t)k * kPiece;
     cudaError_t e = cudaSetDevice(device);
     for (size_t p = k; p < count && e == cudaSuccess; p += threads) {
       unsigned char* h = static_cast<unsigned char*>(host) + p * kPiece;
@@ -88,14 +171,14 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
       const size_t len = std::min(kPiece, bytes - p * kPiece);
       if (down) {
         e = cudaMemcpyAsync(piece, d, len, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaEventRecord(done_[k], stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(done_[k]);
+        if (e == cudaSuccess) e = cudaEventRecord(b.done[k], stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(b.done[k]);
         if (e == cudaSuccess) std::memcpy(h, piece, len);
       } else {
         std::memcpy(piece, h, len);
         e = cudaMemcpyAsync(d, piece, len, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaEventRecord(done_[k], stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(done_[k]);
+        if (e == cudaSuccess) e = cudaEventRecord(b.done[k], stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(b.done[k]);
       }
     }
     err[k] = e;
@@ -110,7 +193,11 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
   work(0);
   for (auto& t : pool) t.join();
   for (int k = started; k < threads; k++) work(k);
-  for (int k = 0; k < threads; k++) check(err[k]);
+  for (int k = 0; k < threads; k++)
+    if (err[k] != cudaSuccess) {
+      cudaStreamSynchronize(stream);  // no copy may still use the pieces
+      check(err[k]);
+    }
 }
 
 void HostCopy::field_to_reference(double* out, const double* field, int64_t stride, int width, const int* order,

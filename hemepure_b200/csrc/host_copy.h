@@ -17,7 +17,7 @@ namespace hb {
 
 class HostCopy {
  public:
-  HostCopy() = default;
+  HostCopy();
   HostCopy(const HostCopy&) = delete;
   HostCopy& operator=(const HostCopy&) = delete;
   ~HostCopy();
@@ -35,15 +35,19 @@ class HostCopy {
                           const int* order_dev, int n, int device, cudaStream_t stream);
 
  private:
-  // 4 MB pinned in all: pinning takes about 0.75 ms a megabyte, once per object.
-  static constexpr int kThreads = 8;
+  // Pinned pieces are the process's, not the object's: pinning takes 1 ms (5 ms as a
+  // fresh allocation), which a handle that is opened, stepped and read once would pay
+  // each time (first pass of a new 257k-site handle, 25 steps and its fields, 9.5 -> 4.4 ms).  A transfer borrows
+  // kThreads pieces; up to kSets of them exist while transfers run side by side, further
+  // transfers are pageable, and all but one set are given back with the last object.
+  static constexpr int kThreads = 8, kSets = 4;
   static constexpr size_t kPiece = (size_t)512 << 10;
   // Up to these sizes one pageable copy: a download gains by its destination's page
   // faults taken in parallel, an upload only by the second copy.
   static constexpr size_t kDirectDown = (size_t)4 << 20, kDirectUp = (size_t)64 << 20;
   void run(void* host, void* dev, size_t bytes, bool down, int device, cudaStream_t stream);
-  unsigned char* pinned_ = nullptr;   // kThreads pieces, made at the first large copy
-  cudaEvent_t done_[kThreads] = {};
+  class Sets;
+  struct Borrowed;
 };
 
 }  // namespace hb

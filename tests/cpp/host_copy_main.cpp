@@ -30,6 +30,9 @@ std::map<void*, size_t> pool_blocks;
 void* own_memory = nullptr;  // a caller's buffer that CUDA knows, of this type
 cudaMemoryType own_type = cudaMemoryTypeUnregistered;
 std::atomic<int> copies{0};     // cudaMemcpyAsync calls
+std::map<const void*, size_t> pinned;
+int pins = 0;                   // allocations and registrations of pinned memory
+bool pinning_fails = false;
 int events_until_failure = -1;  // calls that still succeed before one fails; -1: none fails
 
 cudaError_t note(cudaError_t e) {
@@ -54,7 +57,8 @@ cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; retur
 const char* cudaGetErrorString(cudaError_t) { return "simulated error"; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   std::memset(a, 0, sizeof(*a));
-  a->type = p == own_memory ? own_type : cudaMemoryTypeUnregistered;
+  std::lock_guard<std::mutex> lock(mu);
+  a->type = p == own_memory ? own_type : pinned.count(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t) {
@@ -75,8 +79,25 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   return note(e && of(e)->device == of(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle);
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) { return note(e ? cudaSuccess : cudaErrorInvalidResourceHandle); }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); return cudaSuccess; }
-cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaHostRegister(void* p, size_t n, unsigned) {
+  std::lock_guard<std::mutex> lock(mu);
+  if (pinning_fails) return note(cudaErrorMemoryAllocation);
+  pins++;
+  return note(pinned.emplace(p, n).second ? cudaSuccess : cudaErrorHostMemoryAlreadyRegistered);
+}
+cudaError_t cudaHostUnregister(void* p) {
+  std::lock_guard<std::mutex> lock(mu);
+  return note(pinned.erase(p) ? cudaSuccess : cudaErrorHostMemoryNotRegistered);
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  *p = std::malloc(n);
+  return cudaHostRegister(*p, n, 0);
+}
+cudaError_t cudaFreeHost(void* p) {
+  cudaHostUnregister(p);
+  std::free(p);
+  return cudaSuccess;
+}
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) {
   *p = std::malloc(n);
   std::lock_guard<std::mutex> lock(mu);
@@ -188,6 +209,53 @@ void own_buffers() {
   }
 }
 
+// Handles one after the other pin once; handles side by side pin a bounded number of
+// times and give all but one back; and a field arrives whatever becomes of the pinning.
+void shared_pieces() {
+  FakeStream st{0};
+  Field f(400001, 3);
+  for (int handle = 0; handle < 4; handle++) {
+    hb::HostCopy copy;
+    for (int pass = 0; pass < 2; pass++) {
+      f.fetch(copy, 0, st);
+      require(f.out == f.expect, "field of one of several handles");
+    }
+  }
+  require(pins == 1 && pinned.size() == 1, "handles one after the other pin once");
+  for (int round = 0; round < 3; round++) {
+    std::vector<std::thread> threads;
+    std::atomic<int> right{0};
+    for (int k = 0; k < 8; k++)
+      threads.emplace_back([&] {
+        hb::HostCopy copy;
+        FakeStream own{0};
+        Field g(300007, 3);
+        for (int pass = 0; pass < 3; pass++) {
+          g.fetch(copy, 0, own);
+          right += g.out == g.expect;
+        }
+      });
+    for (auto& t : threads) t.join();
+    require(right == 24, "fields of handles read side by side");
+    require(pinned.size() == 1, "pieces beyond one set are given back");
+  }
+  pinned.clear();  // the context was replaced
+  {
+    hb::HostCopy copy;
+    f.fetch(copy, 0, st);
+    require(f.out == f.expect && pinned.size() == 1, "pieces are pinned again");
+    pinned.clear();
+    pinning_fails = true;
+    for (int pass = 0; pass < 2; pass++) {
+      f.fetch(copy, 0, st);
+      require(f.out == f.expect, "field without pinned memory");
+    }
+    pinning_fails = false;
+    f.fetch(copy, 0, st);
+    require(f.out == f.expect && pinned.size() == 1, "pinned once it can be");
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -196,6 +264,7 @@ int main(int argc, char** argv) {
     if (s == "other_device") other_device();
     else if (s == "event_failure") event_failure();
     else if (s == "own_buffers") own_buffers();
+    else if (s == "shared_pieces") shared_pieces();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());

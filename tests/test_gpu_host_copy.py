@@ -2,6 +2,7 @@
 size that is no multiple of a piece."""
 
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -52,3 +53,27 @@ def test_callers_pinned_array(tmp_path):
     pinned = torch.zeros((sim.n, 19), dtype=torch.float64, pin_memory=True)
     assert lbm.library().hb_get_fs(sim._h, ctypes.cast(pinned.data_ptr(), ctypes.POINTER(ctypes.c_double))) == 0
     assert np.array_equal(pinned.numpy(), sim.GetFOld())
+
+
+def test_two_handles_read_side_by_side(tmp_path):
+    v = vessels.Pipe(20.0, 151)
+    vessels.voxelise(v, str(tmp_path / "c.gmy"))
+    vessels.write_case_xml(str(tmp_path / "c.xml"), "c.gmy", v, vessels.CaseUnits(tau=0.8), 10, [vessels.VelocityBC(0.01)],
+                           [vessels.PressureBC(1.0)])
+    sims = [lbm.LBM(str(tmp_path / "c.xml"), wall="BFL") for _ in range(2)]
+    for k, sim in enumerate(sims):
+        sim.step(3 + k, macro=True)
+    ref = [(*sim.GetPropertyCache(), sim.GetFOld()) for sim in sims]
+    same = [[], []]
+
+    def read(k):
+        for _ in range(4):
+            got = (*sims[k].GetPropertyCache(), sims[k].GetFOld())
+            same[k].append(all(np.array_equal(a, b) for a, b in zip(got, ref[k])))
+
+    threads = [threading.Thread(target=read, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert same == [[True] * 4] * 2
