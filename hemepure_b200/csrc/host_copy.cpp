@@ -207,7 +207,7 @@ void HostCopy::field_to_reference(double* out, const double* field, int64_t stri
   };
   const OnDevice on(device);
   try {
-    SetupPool tmp(device, stream);
+    SetupPool tmp(device, stream, kScratch);
     double* rows = tmp.get<double>((size_t)n * width);
     if (!order_dev) {
       int* o = tmp.get<int>((size_t)n);

@@ -806,7 +806,7 @@ void Solver::set_units(double dt, double dx, const double origin[3]) {
 void Solver::get_fs(double* f) {
   const size_t bytes = (size_t)L_.n * Q * sizeof(double);
   if (mixed()) {
-    SetupPool tmp(opt_.device, stream_);
+    SetupPool tmp(opt_.device, stream_, kScratch);
     double* aos = tmp.get<double>((size_t)L_.n * Q);
     to_aos(false, aos);
     host_copy_.to_host(f, aos, bytes, opt_.device, stream_);
@@ -822,7 +822,7 @@ void Solver::get_fs(double* f) {
 void Solver::set_fs(const double* f) {
   const size_t bytes = (size_t)L_.n * Q * sizeof(double);
   if (mixed()) {
-    SetupPool tmp(opt_.device, stream_);
+    SetupPool tmp(opt_.device, stream_, kScratch);
     double* aos = tmp.get<double>((size_t)L_.n * Q);
     host_copy_.to_device(aos, f, bytes, opt_.device, stream_);
     launch_from_aos_mixed(aos, st2ref_.as<int>(), L_.n, L_.np, opt_.precision, f_[cur_].p, stream_);

@@ -4,6 +4,7 @@
 // Usage: host_copy_main SCENARIO; exits 0 when the scenario's checks hold.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -27,6 +28,7 @@ thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
 std::mutex mu;
 std::map<void*, size_t> pool_blocks;
+size_t pool_used = 0, pool_held = 0;  // bytes given out, and kept by the pool with those
 void* own_memory = nullptr;  // a caller's buffer that CUDA knows, of this type
 cudaMemoryType own_type = cudaMemoryTypeUnregistered;
 std::atomic<int> copies{0};     // cudaMemcpyAsync calls
@@ -102,12 +104,25 @@ cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStrea
   *p = std::malloc(n);
   std::lock_guard<std::mutex> lock(mu);
   pool_blocks[*p] = n;
+  pool_used += n;
+  pool_held = std::max(pool_held, pool_used);
   return cudaSuccess;
 }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) {
   std::lock_guard<std::mutex> lock(mu);
+  pool_used -= pool_blocks[p];
   pool_blocks.erase(p);
   std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v) {
+  std::lock_guard<std::mutex> lock(mu);
+  *static_cast<uint64_t*>(v) = pool_held;
+  return cudaSuccess;
+}
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t keep) {
+  std::lock_guard<std::mutex> lock(mu);
+  pool_held = std::max(pool_used, std::min(pool_held, keep));
   return cudaSuccess;
 }
 }
@@ -256,6 +271,31 @@ void shared_pieces() {
   }
 }
 
+// A transfer's device scratch goes back to what the pool held before it, or to the
+// share it may keep.
+void scratch_given_back() {
+  FakeStream st{0};
+  auto stream = reinterpret_cast<cudaStream_t>(&st);
+  const size_t mb = (size_t)1 << 20;
+  for (size_t before : {(size_t)0, 64 * mb, 1024 * mb}) {
+    pool_held = before;
+    for (size_t bytes : {mb, 100 * mb, 700 * mb, 3000 * mb}) {
+      hb::SetupPool p(0, stream, hb::kScratch);
+      p.get<unsigned char>(bytes);
+    }
+    require(pool_held <= std::max<size_t>(before, hb::kScratchKeep), "scratch is given back");
+    require(pool_held >= before, "what a set-up left in the pool stays");
+  }
+  pool_held = 0;
+  Field f((int)(hb::kScratchKeep / 24) + 1001, 3);
+  hb::HostCopy copy;
+  f.fetch(copy, 0, st);
+  require(f.out == f.expect && pool_held <= hb::kScratchKeep, "a field's scratch is given back");
+  pool_held = 0;
+  { hb::SetupPool p(0, stream); p.get<unsigned char>(700 * mb); }
+  require(pool_held == 700 * mb, "a set-up's memory is kept for the next");
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -265,6 +305,7 @@ int main(int argc, char** argv) {
     else if (s == "event_failure") event_failure();
     else if (s == "own_buffers") own_buffers();
     else if (s == "shared_pieces") shared_pieces();
+    else if (s == "scratch_given_back") scratch_given_back();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());

@@ -2,12 +2,15 @@
 size that is no multiple of a piece."""
 
 import ctypes
+import subprocess
+import sys
 import threading
 
 import numpy as np
 import pytest
 import torch
 
+from conftest import ROOT
 from hemepure_b200 import lbm, vessels
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +80,31 @@ def test_two_handles_read_side_by_side(tmp_path):
     for t in threads:
         t.join()
     assert same == [[True] * 4] * 2
+
+
+SCRATCH = """
+import sys
+import torch
+from hemepure_b200 import lbm
+small, large = (lbm.LBM(x, wall="BFL", precision="fp32", geometry_reader="host") for x in sys.argv[1:3])
+small.SetFs(small.GetFOld())  # the kernels are loaded
+torch.cuda.synchronize()
+before = torch.cuda.mem_get_info()[0]
+large.SetFs(large.GetFOld())
+print(large.n, before - torch.cuda.mem_get_info()[0])
+"""
+
+
+def test_scratch_of_large_distributions_is_given_back(tmp_path):
+    """Distributions of 186 MB go through device scratch of that size, of which the
+    process keeps 128 MB at most (in a process of its own: a set-up on the device
+    leaves the pool larger)."""
+    for name, v in (("s", vessels.Pipe(6.0, 31)), ("l", vessels.Pipe(31.2, 400))):
+        vessels.voxelise(v, str(tmp_path / (name + ".gmy")))
+        vessels.write_case_xml(str(tmp_path / (name + ".xml")), name + ".gmy", v, vessels.CaseUnits(tau=0.8), 10,
+                               [vessels.VelocityBC(0.01)], [vessels.PressureBC(1.0)])
+    r = subprocess.run([sys.executable, "-c", SCRATCH, str(tmp_path / "s.xml"), str(tmp_path / "l.xml")], cwd=ROOT,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    n, kept = map(int, r.stdout.split())
+    assert n * 19 * 8 > 180e6 and kept <= 136 << 20
