@@ -565,14 +565,9 @@ void Batch::get_macro(int slot, double* rho, double* u, double* wss) {
   if (it == members_.end()) throw Error{HB_ERR_ARG, "no such batch member"};
   const BatchMember& m = *it->second;
   if (!m.finished) throw Error{HB_ERR_ARG, "the member has not finished; its fields are filled on its last step"};
-  auto fetch = [&](const DeviceBuffer& field, int width, double* out) {
-    if (out)
-      host_copy_.field_to_reference(out, field.as<double>() + m.site_base, np_, width, m.L.st2ref.data(), nullptr, m.L.n,
-                                    device_, stream_);
-  };
-  fetch(rho_, 1, rho);
-  fetch(u_, 3, u);
-  fetch(wss_, 1, wss);
+  const int64_t at = m.site_base;
+  host_copy_.fields_to_reference({{rho_.as<double>() + at, 1, rho}, {u_.as<double>() + at, 3, u}, {wss_.as<double>() + at, 1, wss}},
+                                 np_, m.L.st2ref.data(), nullptr, m.L.n, device_, stream_);
 }
 
 }  // namespace hb

@@ -200,32 +200,43 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
     }
 }
 
-void HostCopy::field_to_reference(double* out, const double* field, int64_t stride, int width, const int* order,
-                                  const int* order_dev, int n, int device, cudaStream_t stream) {
+void HostCopy::fields_to_reference(std::initializer_list<Field> fields, int64_t stride, const int* order,
+                                   const int* order_dev, int n, int device, cudaStream_t stream) {
   auto check = [](cudaError_t e) {
     if (e != cudaSuccess) throw Error{HB_ERR_CUDA, std::string("field download: ") + cudaGetErrorString(e)};
   };
+  int width = 0;
+  for (const Field& f : fields)
+    if (f.out) width = std::max(width, f.width);
+  if (width == 0 || n <= 0) return;
   const OnDevice on(device);
+  SetupPool tmp(device, stream, kScratch);
+  double* rows = nullptr;
   try {
-    SetupPool tmp(device, stream, kScratch);
-    double* rows = tmp.get<double>((size_t)n * width);
+    rows = tmp.get<double>((size_t)n * width);
     if (!order_dev) {
       int* o = tmp.get<int>((size_t)n);
       check(cudaMemcpyAsync(o, order, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, stream));
       order_dev = o;
     }
-    launch_to_reference(field, stride, width, order_dev, n, rows, stream);
-    check(cudaGetLastError());
-    to_host(out, rows, (size_t)n * width * sizeof(double), device, stream);
-    return;
   } catch (const Error& e) {
     if (e.code != HB_ERR_OOM) throw;
     cudaGetLastError();
+    rows = nullptr;
   }
-  std::vector<double> v((size_t)n);
-  for (int c = 0; c < width; c++) {
-    to_host(v.data(), field + (size_t)c * stride, v.size() * sizeof(double), device, stream);
-    for (int s = 0; s < n; s++) out[(size_t)order[s] * width + c] = v[s];
+  std::vector<double> v(rows ? 0 : (size_t)n);
+  for (const Field& f : fields) {
+    if (!f.out) continue;
+    if (rows) {
+      launch_to_reference(f.field, stride, f.width, order_dev, n, rows, stream);
+      check(cudaGetLastError());
+      to_host(f.out, rows, (size_t)n * f.width * sizeof(double), device, stream);
+      continue;
+    }
+    for (int c = 0; c < f.width; c++) {
+      to_host(v.data(), f.field + (size_t)c * stride, v.size() * sizeof(double), device, stream);
+      for (int s = 0; s < n; s++) f.out[(size_t)order[s] * f.width + c] = v[s];
+    }
   }
 }
 

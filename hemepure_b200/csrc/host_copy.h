@@ -12,6 +12,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <initializer_list>
 
 namespace hb {
 
@@ -25,14 +26,20 @@ class HostCopy {
   void to_host(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream) { run(dst, const_cast<void*>(src), bytes, true, device, stream); }
   void to_device(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream) { run(const_cast<void*>(src), dst, bytes, false, device, stream); }
 
-  // A field of `width` values a site, [width][stride] in storage order on the
-  // device, to `out` as [n][width] in reference order (`order`: storage index to
-  // reference index; `order_dev` the same on the device, or null).  A kernel
-  // reorders it, so that the host only receives it (density, velocity and
-  // stress of 4M sites: 160 ms with the reordering on the host, 12 ms so); with no device memory left
-  // for the reordered copy the host reorders it.
-  void field_to_reference(double* out, const double* field, int64_t stride, int width, const int* order,
-                          const int* order_dev, int n, int device, cudaStream_t stream);
+  // Fields of `width` values a site, [width][stride] in storage order on the device, to
+  // `out` as [n][width] in reference order (`order`: storage index to reference index;
+  // `order_dev` the same on the device, or null: it is then uploaded once for them all).
+  // A kernel reorders them, so that the host only receives them (density, velocity and
+  // stress of 4M sites: 160 ms with the reordering on the host, 12 ms so); with no device
+  // memory left for the reordered copy the host reorders it.  Fields without `out` are
+  // passed over.
+  struct Field {
+    const double* field;
+    int width;
+    double* out;
+  };
+  void fields_to_reference(std::initializer_list<Field> fields, int64_t stride, const int* order, const int* order_dev, int n,
+                           int device, cudaStream_t stream);
 
  private:
   // Pinned pieces are the process's, not the object's: pinning takes 1 ms (5 ms as a

@@ -841,15 +841,13 @@ void Solver::set_fs(const double* f) {
   check(cudaStreamSynchronize(stream_), "set_fs");
 }
 
-void Solver::fetch_field(const double* field, int width, double* out) {
-  host_copy_.field_to_reference(out, field, L_.np, width, L_.st2ref.data(), st2ref_.as<int>(), L_.n, opt_.device, stream_);
+void Solver::fetch_fields(std::initializer_list<HostCopy::Field> fields) {
+  host_copy_.fields_to_reference(fields, L_.np, L_.st2ref.data(), st2ref_.as<int>(), L_.n, opt_.device, stream_);
 }
 
 void Solver::get_macro(double* rho, double* u, double* wss) {
   if (!macro_valid_ || !rho_.p) throw Error{HB_ERR_ARG, "no step has filled the macroscopic caches (pass HB_STEP_MACRO)"};
-  if (rho) fetch_field(rho_.as<double>(), 1, rho);
-  if (u) fetch_field(u_.as<double>(), 3, u);
-  if (wss) fetch_field(wss_.as<double>(), 1, wss);
+  fetch_fields({{rho_.as<double>(), 1, rho}, {u_.as<double>(), 3, u}, {wss_.as<double>(), 1, wss}});
 }
 
 int Solver::stress_len(int field) {
@@ -880,7 +878,7 @@ void Solver::get_stress(int field, double* out) {
   a.pi = pi_.as<double>();
   launch_stress_field(a, field, stress_out_.as<double>(), stream_);
   check(cudaGetLastError(), "stress field launch");
-  fetch_field(stress_out_.as<double>(), k, out);
+  fetch_fields({{stress_out_.as<double>(), k, out}});
 }
 
 void Solver::moment_sums(double out[4]) {

@@ -128,7 +128,7 @@ class Solver {
   void launch_wk3(cudaStream_t st);
   int step_launches(bool macro) const;
   void to_aos(bool use_prev, double* dev_aos);
-  void fetch_field(const double* field, int width, double* out);
+  void fetch_fields(std::initializer_list<HostCopy::Field> fields);
 
   LatticeTables t_;
   hb_params p_;

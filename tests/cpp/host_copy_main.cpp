@@ -157,7 +157,7 @@ struct Field {
   }
   void fetch(hb::HostCopy& c, int device, FakeStream& st) {
     std::fill(out.begin(), out.end(), -1.0);
-    c.field_to_reference(out.data(), storage.data(), n, width, order.data(), order.data(), n, device, reinterpret_cast<cudaStream_t>(&st));
+    c.fields_to_reference({{storage.data(), width, out.data()}}, n, order.data(), order.data(), n, device, reinterpret_cast<cudaStream_t>(&st));
   }
 };
 
@@ -296,6 +296,19 @@ void scratch_given_back() {
   require(pool_held == 700 * mb, "a set-up's memory is kept for the next");
 }
 
+// Several fields of one member: their order crosses to the device once.
+void one_order() {
+  FakeStream st{0};
+  const int n = 10007;
+  Field a(n, 1), b(n, 3), c(n, 1);
+  hb::HostCopy copy;
+  copies = 0;
+  copy.fields_to_reference({{a.storage.data(), 1, a.out.data()}, {b.storage.data(), 3, b.out.data()}, {c.storage.data(), 1, nullptr}}, n,
+                           a.order.data(), nullptr, n, 0, reinterpret_cast<cudaStream_t>(&st));
+  require(a.out == a.expect && b.out == b.expect, "fields by an uploaded order");
+  require(copies == 3, "one upload of the order and a download of each field asked for");
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -306,6 +319,7 @@ int main(int argc, char** argv) {
     else if (s == "own_buffers") own_buffers();
     else if (s == "shared_pieces") shared_pieces();
     else if (s == "scratch_given_back") scratch_given_back();
+    else if (s == "one_order") one_order();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());
