@@ -41,10 +41,9 @@ struct WK3Dev {           // InOutLetWK3 / InOutLetWK2 state
   int pad[2];
 };
 
-// What a step launcher launches (`which`) of a steady-state step: the plain bulk
-// sites, the boundary records without iolet links (and the GZS wall links), the
-// boundary records with them.  The first step of a state and the output steps
-// always launch everything.
+// What a step launcher launches (`which`): the plain bulk sites, the boundary records
+// without iolet links (and the GZS wall links), the boundary records with them.  The
+// first step of a state and the output steps take all boundary records together.
 constexpr int kLaunchBulk = 1, kLaunchWallRecords = 4, kLaunchIoletRecords = 8;
 constexpr int kLaunchBoundary = kLaunchWallRecords | kLaunchIoletRecords, kLaunchAll = kLaunchBulk | kLaunchBoundary;
 

@@ -538,6 +538,15 @@ void Solver::pre_receive(bool macro, int which, bool stress) {
     launch(a, macro, which & ~kLaunchIoletRecords, stream_);
     check(cudaStreamWaitEvent(stream_, join_, 0), "join");
     wk_beside_ = false;
+  } else if ((direct_ || macro) && (which & kLaunchBulk) && (which & kLaunchBoundary)) {
+    // These forms have no kernel of all kinds of work: the bulk sites and the boundary
+    // beside each other.
+    check(cudaEventRecord(fork_, stream_), "fork");
+    check(cudaStreamWaitEvent(side_, fork_, 0), "fork");
+    launch(a, macro, kLaunchBoundary, side_);
+    check(cudaEventRecord(join_, side_), "join");
+    launch(a, macro, kLaunchBulk, stream_);
+    check(cudaStreamWaitEvent(stream_, join_, 0), "join");
   } else {
     launch(a, macro, which, stream_);
   }
@@ -547,9 +556,9 @@ void Solver::pre_receive(bool macro, int which, bool stress) {
 }
 
 // Kernels of one step: one for a steady-state step (two with the iolet records
-// beside it), else one per kind of work.
+// beside it), else the bulk sites' and the boundary's.
 int Solver::step_launches(bool macro) const {
-  if (direct_ || macro) return 1 + (L_.G > 0 ? 1 : 0) + (iol_n_ > 0 ? 1 : 0) + (gzs_n_ > 0 ? 1 : 0);
+  if (direct_ || macro) return 1 + (L_.G > 0 ? 1 : 0);
   return 1 + (wk_beside_ && L_.G > L_.kind_start[2] ? 1 : 0);
 }
 

@@ -136,7 +136,7 @@ class Solver {
   hb_options opt_;
   Layout L_;
   cudaStream_t stream_ = nullptr;
-  cudaStream_t side_ = nullptr;   // Windkessel update and iolet records, beside the other sites
+  cudaStream_t side_ = nullptr;   // Windkessel update and iolet records, or the boundary of an output step, beside the other sites
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   cudaEvent_t fork_ = nullptr, join_ = nullptr;
 

@@ -57,6 +57,16 @@ inline StepTiles step_tiles(const StepArgs& a, int which, int resident) {
   return t;
 }
 
+// The boundary on its own: iolet links, GZS wall links, then every record (as `io`).
+inline StepTiles boundary_tiles(const StepArgs& a) {
+  StepTiles t{};
+  auto blocks = [](int64_t n) { return (int)((n + kStepBlock - 1) / kStepBlock); };
+  t.links = blocks(a.iol_n);
+  t.gzs = blocks(a.gzs_n);
+  t.io = blocks(a.gen.G);
+  return t;
+}
+
 // Wait for the step that wrote this step's input, then let the next step's blocks
 // be launched as this one's blocks leave (a no-op in a plain launch).  Only
 // constant tables may be read before it.

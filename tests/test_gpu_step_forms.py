@@ -52,3 +52,15 @@ def test_shifted_forms_follow_the_oracle(tmp_path, precision, wall, radius, leng
     assert orc.run(40, macro=True) == 0
     u, ref = gpu.GetPropertyCache()[1], orc.macro()[1]
     assert np.abs(u - ref).max() <= U_TOL[precision] * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("wall", ["GZS", "BFL"])
+def test_first_and_output_steps_take_two_kernels(tmp_path, precision, wall):
+    """One for the plain bulk sites and one for the boundary, which run side by side
+    (a kernel for each kind of boundary work one after the other made an output step a
+    quarter longer than before them); a step in between is one launch."""
+    sim = lbm.LBM(pipe_case(tmp_path, 7.6, 33, True, True), kernel="TRT", wall=wall, precision=precision)
+    for macro, launches in ((False, 2), (False, 1), (True, 2), (False, 1)):
+        sim.step(1, macro=macro)
+        assert sim.last_step_timing()[1] == launches
