@@ -156,7 +156,7 @@ void HostCopy::run(void* host, void* dev, size_t bytes, bool down, int device, c
   if (!pieces) {
     check(cudaMemcpyAsync(down ? host : dev, down ? dev : host, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
                           stream));
-    check(cudaStreamSynchronize(stream));
+    if (down) check(cudaStreamSynchronize(stream));
     return;
   }
   const size_t count = (bytes + kPiece - 1) / kPiece;

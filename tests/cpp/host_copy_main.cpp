@@ -32,6 +32,7 @@ size_t pool_used = 0, pool_held = 0;  // bytes given out, and kept by the pool w
 void* own_memory = nullptr;  // a caller's buffer that CUDA knows, of this type
 cudaMemoryType own_type = cudaMemoryTypeUnregistered;
 std::atomic<int> copies{0};     // cudaMemcpyAsync calls
+std::atomic<int> waits{0};      // cudaStreamSynchronize calls
 std::map<const void*, size_t> pinned;
 int pins = 0;                   // allocations and registrations of pinned memory
 bool pinning_fails = false;
@@ -70,7 +71,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kin
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { waits++; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
   if (events_until_failure >= 0 && events_until_failure-- == 0) return note(cudaErrorMemoryAllocation);
   *e = reinterpret_cast<cudaEvent_t>(new FakeEvent{current});
@@ -309,6 +310,19 @@ void one_order() {
   require(copies == 3, "one upload of the order and a download of each field asked for");
 }
 
+// A small upload is followed by its caller's kernel and wait: it does not wait itself.
+// A download is done when its call returns.
+void small_copies() {
+  FakeStream st{0};
+  auto stream = reinterpret_cast<cudaStream_t>(&st);
+  std::vector<double> a(1000, 1.5), b(1000);
+  hb::HostCopy copy;
+  copy.to_device(b.data(), a.data(), a.size() * sizeof(double), 0, stream);
+  require(a == b && waits == 0, "a small upload does not wait");
+  copy.to_host(b.data(), a.data(), a.size() * sizeof(double), 0, stream);
+  require(waits == 1, "a small download waits once");
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -320,6 +334,7 @@ int main(int argc, char** argv) {
     else if (s == "shared_pieces") shared_pieces();
     else if (s == "scratch_given_back") scratch_given_back();
     else if (s == "one_order") one_order();
+    else if (s == "small_copies") small_copies();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());
