@@ -225,10 +225,8 @@ void Batch::write_member_tables(const BatchMember& m) {
     put(g_cpl_, m.gen_base, cpl.data(), G, stream_);
     put(g_lat_, m.gen_base, lat.data(), G, stream_);
     put_rows(g_src_, cap_gen_, m.gen_base, src.data(), G, 18, stream_);
-    std::vector<float> coef(L.g_q);
-    if (m.wall == kBFL)
-      for (float& q : coef) q = bfl_coefficient(q);
-    put_rows(g_q_, cap_gen_, m.gen_base, coef.data(), G, 18, stream_);
+    put_rows(g_q_, cap_gen_, m.gen_base, L.g_q.data(), G, 18, stream_);
+    if (m.wall == kBFL) launch_bfl_coefficients(g_q_.as<float>() + m.gen_base, cap_gen_, G, stream_);
     put_rows(g_nrm_, cap_gen_, m.gen_base, L.g_nrm.data(), G, 3, stream_);
     put_rows(g_xyz_, cap_gen_, m.gen_base, L.g_xyz.data(), G, 3, stream_);
     std::vector<int> iol;

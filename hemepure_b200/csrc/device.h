@@ -132,6 +132,8 @@ void launch_step_mixed(const StepArgs& a, int precision, const void* fin, void* 
 void launch_to_aos_mixed(const StepArgs& a, int precision, const void* fin, const float* gin, int wall, bool gather,
                          const int* st2ref, double* aos, void* stream);
 void launch_from_aos_mixed(const double* aos, const int* st2ref, int n, int64_t np, int precision, void* out, void* stream);
+// The BFL coefficients of the shifted forms in place of the cut distances (kernels_mixed.cu).
+void launch_bfl_coefficients(float* q, int64_t pitch, int n, void* stream);
 // Conserved sums (density, momentum x/y/z) over n sites in FP64, deterministic:
 // one partial per block of kSumSitesPerBlock sites in `scratch` (4 doubles per
 // block), then the partials in block order into `out` (4 doubles, device).

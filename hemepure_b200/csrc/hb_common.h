@@ -47,13 +47,6 @@ enum IoletKind { kCosine = 0, kWK3 = 1, kParabolic = 2, kWK2 = 3, kFile = 4, kFi
 // Velocity iolets take the Ladd streamer; the others the Nash zeroth-order pressure streamer.
 HB_HD constexpr bool is_velocity_iolet(int kind) { return kind == kParabolic || kind == kFileVelocity || kind == kWomersley; }
 
-// Coefficient of the shifted forms' BFL rule for cut distance q, from
-// (f*_d + (2q-1) f*_i) / (2q) = f*_d + c (f*_i - f*_d), c = 1 - 1/(2q), for q >= 1/2 and
-// 2q f*_d + (1-2q) f_d = f*_d + |c| (f_d - f*_d), c = -(1-2q), otherwise.
-inline float bfl_coefficient(float q) {
-  return q < 0.5f ? (float)-(1.0 - 2.0 * (double)q) : (float)(1.0 - 1.0 / (2.0 * (double)q));
-}
-
 // Host-side error carrying one of the HB_ERR_* codes.
 struct Error {
   int code;

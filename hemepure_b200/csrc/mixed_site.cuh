@@ -333,7 +333,7 @@ __device__ __forceinline__ void load_sources_m(const StepArgs& a, const LinksM& 
 // (s + run offset for a record that follows its run, else its pull table).  The
 // BFL correction of wall links follows as a predicated step: both of its rules
 // (gather_links, f64_site.cuh) are g*_d + |c| (X - g*_d) with the coefficient c of
-// bfl_coefficient laid out once per link, so the kernels divide by nothing here.
+// k_bfl_coefficients laid out once per link, so the kernels divide by nothing here.
 template <class S, bool IO = true>
 __device__ __forceinline__ void gather_links_m(const StepArgs& a, const MixArgs& m, const LinksM& l, int s, const int* src,
                                                bool bfl, float* g) {

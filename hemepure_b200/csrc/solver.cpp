@@ -192,12 +192,10 @@ void Solver::upload() {
   upload_vec(g_wall_, L_.g_wall, tot);
   upload_vec(g_iolet_, L_.g_iolet, tot);
   upload_vec(g_src_, L_.g_src, tot);
+  upload_vec(g_q_, L_.g_q, tot);
   if (mixed() && opt_.wall == kBFL) {
-    std::vector<float> coef(L_.g_q);
-    for (float& q : coef) q = bfl_coefficient(q);
-    upload_vec(g_q_, coef, tot);
-  } else {
-    upload_vec(g_q_, L_.g_q, tot);
+    launch_bfl_coefficients(g_q_.as<float>(), L_.G, L_.G, stream_);
+    check(cudaGetLastError(), "BFL coefficients");
   }
   upload_vec(g_nrm_, L_.g_nrm, tot);
   upload_vec(g_io_, L_.g_io, tot);
