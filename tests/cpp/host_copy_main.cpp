@@ -28,6 +28,7 @@ thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
 std::mutex mu;
 std::map<void*, size_t> pool_blocks;
+bool pool_empty = false;              // no device memory to be had
 size_t pool_used = 0, pool_held = 0;  // bytes given out, and kept by the pool with those
 void* own_memory = nullptr;  // a caller's buffer that CUDA knows, of this type
 cudaMemoryType own_type = cudaMemoryTypeUnregistered;
@@ -102,6 +103,7 @@ cudaError_t cudaFreeHost(void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) {
+  if (pool_empty) return note(cudaErrorMemoryAllocation);
   *p = std::malloc(n);
   std::lock_guard<std::mutex> lock(mu);
   pool_blocks[*p] = n;
@@ -323,6 +325,25 @@ void small_copies() {
   require(waits == 1, "a small download waits once");
 }
 
+// Without device memory for the reordered copy the host reorders the fields, to the
+// same values; sizes on both sides of a piece and of the set of pieces.
+void no_device_memory() {
+  FakeStream st{0};
+  for (int n : {1, 65535, 65536, 65537, 600011}) {
+    hb::HostCopy copy;
+    Field a(n, 3), b(n, 1);
+    for (bool empty : {false, true}) {
+      pool_empty = empty;
+      std::fill(a.out.begin(), a.out.end(), -1.0);
+      std::fill(b.out.begin(), b.out.end(), -1.0);
+      copy.fields_to_reference({{a.storage.data(), 3, a.out.data()}, {b.storage.data(), 1, b.out.data()}}, n, a.order.data(), nullptr, n, 0,
+                               reinterpret_cast<cudaStream_t>(&st));
+      require(a.out == a.expect && b.out == b.expect, empty ? "fields reordered on the host" : "fields reordered on the device");
+    }
+    pool_empty = false;
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -335,6 +356,7 @@ int main(int argc, char** argv) {
     else if (s == "scratch_given_back") scratch_given_back();
     else if (s == "one_order") one_order();
     else if (s == "small_copies") small_copies();
+    else if (s == "no_device_memory") no_device_memory();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());

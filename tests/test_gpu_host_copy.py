@@ -21,7 +21,8 @@ C = np.array([(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1)
 
 
 @pytest.mark.parametrize("precision,eps", [("fp64", 2.0 ** -53), ("fp32", 2.0 ** -24)])
-@pytest.mark.parametrize("radius,length", [(6.0, 31), (20.0, 151)])  # u below and above a piece
+# u below and above the size that goes in pieces, and f above it in both directions (75 MB up)
+@pytest.mark.parametrize("radius,length", [(6.0, 31), (20.0, 151), (22.3, 317)])
 def test_fields_arrive_in_reference_order(tmp_path, precision, eps, radius, length):
     v = vessels.Pipe(radius, length)
     vessels.voxelise(v, str(tmp_path / "c.gmy"))
@@ -31,6 +32,7 @@ def test_fields_arrive_in_reference_order(tmp_path, precision, eps, radius, leng
     rng = np.random.default_rng(3)
     w = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12)
     f = w * (1.0 + 1e-3 * rng.standard_normal((sim.n, 19)))
+    assert f.nbytes % (512 << 10) and (length < 300 or f.nbytes > 64 << 20)
     sim.SetFs(f)
     got = sim.GetFOld()
     # FP64 storage is exact; FP32 rounds the deviation from w, at most 5e-3 w.

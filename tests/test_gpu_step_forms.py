@@ -10,9 +10,12 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
-# FP32: each step rounds a deviation of order 1e-2 to 2^-24 of itself and 40 steps add
-# at most linearly, against a velocity of order 1e-3; FP16 storage likewise with 2^-11.
-U_TOL = {"fp32": 40 * 2.0 ** -24 * 1e-2 / 1e-3 * 4, "fp16": 40 * 2.0 ** -11 * 1e-2 / 1e-3 * 4}
+# Largest difference over the field's largest value.  Storing a deviation rounds it to
+# 2^-24 (FP32) or 2^-11 (FP16) of itself at most, every step; such errors are unbiased and
+# add like a random walk.  Twice that: the collision rounds too, and wall shear stress is
+# a difference of such values.  (Seen: 0.66 and 0.16 of it.  Bounce-back in place of a BFL
+# or GZS wall moves wall velocities by 0.16 and more, BFL in place of GZS by 0.008.)
+TOL = {"fp32": 2 * np.sqrt(40) * 2.0 ** -24, "fp16": 2 * np.sqrt(40) * 2.0 ** -11}
 
 
 def pipe_case(tmp, radius, length, velocity, trt):
@@ -45,13 +48,19 @@ def test_step_forms_bit_exact(tmp_path, radius, length, kernel, wall, velocity):
 @pytest.mark.parametrize("wall", ["GZS", "BFL", "SBB"])
 @pytest.mark.parametrize("radius,length", [(2.3, 5), (7.6, 33), (6.2, 70)])
 def test_shifted_forms_follow_the_oracle(tmp_path, precision, wall, radius, length):
-    """Pairs of sites across run ends, partial tiles and boundary records."""
+    """Velocity everywhere, and wall shear stress at the wall records on its own, so
+    that a fault of the boundary links alone shows."""
     xml = pipe_case(tmp_path, radius, length, True, True)
     gpu, orc = lbm.LBM(xml, kernel="TRT", wall=wall, precision=precision), O.Simulation(xml, "TRT", wall)
     gpu.step(40, macro=True)
     assert orc.run(40, macro=True) == 0
-    u, ref = gpu.GetPropertyCache()[1], orc.macro()[1]
-    assert np.abs(u - ref).max() <= U_TOL[precision] * np.abs(ref).max()
+    (_, u, w), (_, u_ref, w_ref) = gpu.GetPropertyCache(), orc.macro()
+    at = w_ref < 1e300
+    assert at.any() and np.array_equal(at, w < 1e300)
+    err = {"u": np.abs(u - u_ref).max() / np.abs(u_ref).max(), "u_wall": np.abs(u - u_ref)[at].max() / np.abs(u_ref[at]).max(),
+           "wss": np.abs(w - w_ref)[at].max() / w_ref[at].max()}
+    print(f"{precision} {wall} radius {radius}: {err}")
+    assert max(err.values()) <= TOL[precision], err
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
