@@ -19,8 +19,9 @@ back the stability word, with a host synchronisation).
 The CPU baseline and the reference arm (`--impl reference`) run HemePure's
 own code, compiled from its sources into oracle/_ref (single-rank: no MPI
 library exists on these machines), as one copy of the lattice per host core
-side by side, on a bounded number of steps; where those executables are not
-built, the oracle's C restatement runs on all host threads instead.
+side by side, on a bounded number of steps.  Where those executables are not
+built, the reference arm says so and the CPU baseline is the oracle's C
+restatement on all host threads (`kind: port`).
 """
 
 from __future__ import annotations
@@ -266,10 +267,13 @@ def main():
 
     if args.impl == "reference":
         # HemePure itself, compiled from its own sources (oracle/_ref), one copy per
-        # host core; its C restatement on all host threads where it is not built.
+        # host core.
         base = reference_cpu(xml, kernel, wall, n_sites, budget_s=60.0, max_steps=args.steps, warmup=warmup)
         if base is None:
-            base = cpu_baseline(xml, kernel, wall, n_sites, budget_s=120.0)
+            print(json.dumps({"impl": "reference", "unavailable":
+                              "HemePure's executables are not built here (oracle/_ref), nor are its sources on this machine"}),
+                  flush=True)
+            return
         v = base["value"]
         line = {"impl": "reference", "metric": METRIC, "value": v, "unit": "MLUPS", "n_gpus": args.gpus,
                 "steps": args.steps, "warmup": warmup, "ms_per_step": n_sites / (v * 1e6) * 1e3,

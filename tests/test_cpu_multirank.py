@@ -61,3 +61,17 @@ def test_reference_arm_on_a_nonzero_rank_exits_without_work():
     r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--gpus", "2"],
                        capture_output=True, text=True, env=env, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == ""
+
+
+def test_reference_arm_without_the_reference_says_so(tmp_path):
+    """The arm measures HemePure or nothing: no restatement of this repository's."""
+    import json
+    from oracle import reference as R
+    xml, _ = bench.make_workload("pipe_r8", str(tmp_path / "w"))
+    if R.available(R.combo_for(xml, "LBGK", "SBB")):
+        import pytest
+        pytest.skip("HemePure's executables are built here")
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--workload", "pipe_r8",
+                        "--steps", "2", "--case-dir", str(tmp_path)], capture_output=True, text=True, timeout=120)
+    line = json.loads(r.stdout)
+    assert r.returncode == 0 and line["impl"] == "reference" and line["unavailable"] and "value" not in line
