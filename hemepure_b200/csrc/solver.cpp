@@ -193,10 +193,6 @@ void Solver::upload() {
   upload_vec(g_iolet_, L_.g_iolet, tot);
   upload_vec(g_src_, L_.g_src, tot);
   upload_vec(g_q_, L_.g_q, tot);
-  if (mixed() && opt_.wall == kBFL) {
-    launch_bfl_coefficients(g_q_.as<float>(), L_.G, L_.G, stream_);
-    check(cudaGetLastError(), "BFL coefficients");
-  }
   upload_vec(g_nrm_, L_.g_nrm, tot);
   upload_vec(g_io_, L_.g_io, tot);
   upload_vec(g_cpl_, L_.g_cpl, tot);
@@ -342,6 +338,14 @@ void Solver::upload() {
   *status_host_ = 0;
   check(cudaMemset(status_.p, 0, sizeof(int)), "cudaMemset");
   dev_bytes_ = tot;
+
+  // A pageable upload returns once it is staged, and stream_ does not wait for the
+  // default stream: the tables have to have arrived before a kernel reads them.
+  check(cudaStreamSynchronize(cudaStreamLegacy), "table upload");
+  if (mixed() && opt_.wall == kBFL) {
+    launch_bfl_coefficients(g_q_.as<float>(), L_.G, L_.G, stream_);
+    check(cudaGetLastError(), "BFL coefficients");
+  }
 
   // Equilibrium initial condition in direct form.
   double feq[Q];
