@@ -4,7 +4,7 @@
 #include <sys/mman.h>
 
 #include <algorithm>
-#include <cstdlib>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -65,13 +65,10 @@ class HostCopy::Sets {
         made_++;
       }
     }
-    if (!p) {
-      p = static_cast<unsigned char*>(std::aligned_alloc(kHugePage, kBytes));
-      if (p) madvise(p, kBytes, MADV_HUGEPAGE);  // two pages to pin instead of a thousand
-    }
+    if (!p) p = map();
     if (p && !pinned(p) && cudaHostRegister(p, kBytes, cudaHostRegisterPortable) != cudaSuccess) {
       cudaGetLastError();
-      std::free(p);
+      munmap(p, kBytes);
       p = nullptr;
     }
     if (!p) {
@@ -93,13 +90,26 @@ class HostCopy::Sets {
     if (--users_ > 0) return;
     for (; free_.size() > 1; free_.pop_back(), made_--) {
       if (cudaHostUnregister(free_.back()) != cudaSuccess) cudaGetLastError();
-      std::free(free_.back());
+      munmap(free_.back(), kBytes);
     }
   }
 
  private:
+  Sets() { free_.reserve(kSets); }  // give() runs on every path out of a transfer
   static constexpr size_t kHugePage = (size_t)2 << 20, kBytes = kThreads * kPiece;
-  static_assert(kBytes % kHugePage == 0, "aligned_alloc takes a multiple of the alignment");
+  // Two huge pages to pin instead of a thousand, and none shared with a child process:
+  // CUDA would go on copying from and to a page that the next write leaves to the child.
+  static unsigned char* map() {
+    void* m = mmap(nullptr, kBytes + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == MAP_FAILED) return nullptr;
+    unsigned char* lo = static_cast<unsigned char*>(m);
+    const size_t head = (kHugePage - (uintptr_t)lo % kHugePage) % kHugePage, tail = kHugePage - head;
+    if (head) munmap(lo, head);
+    if (tail) munmap(lo + head + kBytes, tail);
+    madvise(lo + head, kBytes, MADV_HUGEPAGE);
+    madvise(lo + head, kBytes, MADV_DONTFORK);
+    return lo + head;
+  }
   static bool pinned(const void* p) {
     cudaPointerAttributes attr{};
     if (cudaPointerGetAttributes(&attr, p) == cudaSuccess) return attr.type == cudaMemoryTypeHost;

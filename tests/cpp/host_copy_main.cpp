@@ -9,8 +9,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <fstream>
 #include <map>
 #include <mutex>
+#include <sstream>
 #include <string>
 #include <thread>
 #include <vector>
@@ -344,6 +346,31 @@ void no_device_memory() {
   }
 }
 
+// Whether the mapping that holds `p` is left out of a child process ("dc" of smaps).
+bool left_out_of_children(const void* p) {
+  std::ifstream in("/proc/self/smaps");
+  std::string line;
+  bool here = false;
+  while (std::getline(in, line)) {
+    unsigned long lo, hi;
+    if (std::sscanf(line.c_str(), "%lx-%lx ", &lo, &hi) == 2) here = lo <= (unsigned long)p && (unsigned long)p < hi;
+    if (here && line.rfind("VmFlags:", 0) == 0) return line.find(" dc") != std::string::npos;
+  }
+  return false;
+}
+
+// A child process shares no piece with its parent: a piece written after a fork would
+// otherwise move to another page than the one CUDA copies from.
+void fork_safe() {
+  FakeStream st{0};
+  Field f(400001, 3);
+  hb::HostCopy copy;
+  f.fetch(copy, 0, st);
+  require(f.out == f.expect && pinned.size() == 1, "a field in pieces");
+  const unsigned char* p = static_cast<const unsigned char*>(pinned.begin()->first);
+  require(left_out_of_children(p) && left_out_of_children(p + pinned.begin()->second - 1), "pieces are left out of child processes");
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -357,6 +384,7 @@ int main(int argc, char** argv) {
     else if (s == "one_order") one_order();
     else if (s == "small_copies") small_copies();
     else if (s == "no_device_memory") no_device_memory();
+    else if (s == "fork_safe") fork_safe();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());
