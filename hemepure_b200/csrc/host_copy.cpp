@@ -52,17 +52,21 @@ class HostCopy::Sets {
     return *s;
   }
   // A set for one transfer; null without memory to pin, or with kSets lent already.
+  // The sets take turns, another one joining after every kTurns transfers: the device
+  // writes faster into memory that no core has read of late.
   unsigned char* take() {
     unsigned char* p = nullptr;
     {
       std::lock_guard<std::mutex> lock(mu_);
-      if (!free_.empty()) {
-        p = free_.back();
-        free_.pop_back();
-      } else if (made_ == kSets) {
-        return nullptr;
-      } else {
+      const bool grow = free_.empty() || made_ < 1 + taken_ / kTurns;
+      taken_ = std::min(taken_ + 1, kSets * kTurns);
+      if (grow && made_ < kSets) {
         made_++;
+      } else if (!free_.empty()) {
+        p = free_.front();
+        free_.erase(free_.begin());
+      } else {
+        return nullptr;
       }
     }
     if (!p) p = map();
@@ -74,6 +78,11 @@ class HostCopy::Sets {
     if (!p) {
       std::lock_guard<std::mutex> lock(mu_);
       made_--;
+      taken_ = 0;
+      if (!free_.empty()) {
+        p = free_.front();
+        free_.erase(free_.begin());
+      }
     }
     return p;
   }
@@ -88,6 +97,7 @@ class HostCopy::Sets {
   void leave() {
     std::lock_guard<std::mutex> lock(mu_);
     if (--users_ > 0) return;
+    taken_ = 0;
     for (; free_.size() > 1; free_.pop_back(), made_--) {
       if (cudaHostUnregister(free_.back()) != cudaSuccess) cudaGetLastError();
       munmap(free_.back(), kBytes);
@@ -118,7 +128,7 @@ class HostCopy::Sets {
   }
   std::mutex mu_;
   std::vector<unsigned char*> free_;
-  int made_ = 0, users_ = 0;
+  int made_ = 0, users_ = 0, taken_ = 0;
 };
 
 // A set and the events of one transfer.

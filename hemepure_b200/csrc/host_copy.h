@@ -46,10 +46,13 @@ class HostCopy {
  private:
   // Pinned pieces are the process's, not the object's: pinning takes 1 ms (5 ms as a
   // fresh allocation), which a handle that is opened, stepped and read once would pay
-  // each time (first pass of a new 257k-site handle, 25 steps and its fields, 9.5 -> 4.4 ms).  A transfer borrows
-  // kThreads pieces; up to kSets of them exist while transfers run side by side, further
-  // transfers are pageable, and all but one set are given back with the last object.
-  static constexpr int kThreads = 8, kSets = 4;
+  // each time (first pass of a new 257k-site handle, 25 steps and its fields, 9.5 -> 4.4
+  // ms).  A transfer borrows a set of kThreads pieces; further transfers beside kSets of
+  // them are pageable.  A set that the cores have just read is slow to write again
+  // (a 4.6 MB field 0.50 ms with one set, 0.45, 0.38, 0.33 with two to four in turn), so
+  // every kTurns transfers one more joins, up to kSets; all but one are given back with
+  // the last object.
+  static constexpr int kThreads = 8, kSets = 4, kTurns = 8;
   static constexpr size_t kPiece = (size_t)512 << 10;
   // Up to these sizes one pageable copy: a download gains by its destination's page
   // faults taken in parallel, an upload only by the second copy.

@@ -371,6 +371,28 @@ void fork_safe() {
   require(left_out_of_children(p) && left_out_of_children(p + pinned.begin()->second - 1), "pieces are left out of child processes");
 }
 
+// A handle that goes on reading has its transfers take turns on a bounded number of
+// sets, whether or not one could not be pinned, and leaves one.
+void sets_in_turn() {
+  FakeStream st{0};
+  Field f(200003, 3);
+  for (bool fails : {false, true}) {
+    hb::HostCopy copy;
+    size_t most = 0;
+    for (int pass = 0; pass < 60; pass++) {
+      pinning_fails = fails && pass > 12;
+      copies = 0;
+      f.fetch(copy, 0, st);
+      require(f.out == f.expect && copies > 1, "a field in pieces by sets in turn");
+      require(pinned.size() >= most, "no set is given up under way");
+      most = pinned.size();
+    }
+    require(most == (fails ? 2 : 4), "sets in turn");
+  }
+  pinning_fails = false;
+  require(pinned.size() == 1, "one set is kept");
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -385,6 +407,7 @@ int main(int argc, char** argv) {
     else if (s == "small_copies") small_copies();
     else if (s == "no_device_memory") no_device_memory();
     else if (s == "fork_safe") fork_safe();
+    else if (s == "sets_in_turn") sets_in_turn();
     else return 2;
   } catch (const hb::Error& e) {
     std::fprintf(stderr, "error %d: %s\n", e.code, e.msg.c_str());

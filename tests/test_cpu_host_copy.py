@@ -20,7 +20,7 @@ def host_copy(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["other_device", "event_failure", "own_buffers", "shared_pieces", "scratch_given_back", "one_order",
-                                      "small_copies", "no_device_memory", "fork_safe"])
+                                      "small_copies", "no_device_memory", "fork_safe", "sets_in_turn"])
 def test_host_copy(host_copy, scenario):
     r = subprocess.run([host_copy, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr
