@@ -141,6 +141,7 @@ Solver::Solver(LatticeTables tables, const hb_params& params, const hb_options& 
   int prio_lo = 0, prio_hi = 0;
   check(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi), "cudaDeviceGetStreamPriorityRange");
   check(cudaStreamCreateWithPriority(&side_, cudaStreamNonBlocking, prio_hi), "cudaStreamCreate");
+  check(cudaStreamCreateWithFlags(&boundary_, cudaStreamNonBlocking), "cudaStreamCreate");
   check(cudaEventCreate(&ev0_), "cudaEventCreate");
   check(cudaEventCreate(&ev1_), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
@@ -152,11 +153,13 @@ Solver::~Solver() {
   if (stream_) cudaStreamSynchronize(stream_);
   if (xev_) cudaEventDestroy(xev_);
   if (side_) cudaStreamSynchronize(side_);
+  if (boundary_) cudaStreamSynchronize(boundary_);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   if (fork_) cudaEventDestroy(fork_);
   if (join_) cudaEventDestroy(join_);
   if (side_) cudaStreamDestroy(side_);
+  if (boundary_) cudaStreamDestroy(boundary_);
   if (stream_) cudaStreamDestroy(stream_);
   if (status_host_) cudaFreeHost(status_host_);
   if (host_rows_) cudaFreeHost(host_rows_);
@@ -542,11 +545,13 @@ void Solver::pre_receive(bool macro, int which, bool stress) {
     wk_beside_ = false;
   } else if ((direct_ || macro) && (which & kLaunchBulk) && (which & kLaunchBoundary)) {
     // These forms have no kernel of all kinds of work: the bulk sites and the boundary
-    // beside each other.
+    // beside each other.  On a stream of its own: with the Windkessel update's stream
+    // in use here too, more of the steady steps after it ran slow (187k-site GZS
+    // bifurcation, 300 steps and an output: 6.83 ms a pass against 6.64).
     check(cudaEventRecord(fork_, stream_), "fork");
-    check(cudaStreamWaitEvent(side_, fork_, 0), "fork");
-    launch(a, macro, kLaunchBoundary, side_);
-    check(cudaEventRecord(join_, side_), "join");
+    check(cudaStreamWaitEvent(boundary_, fork_, 0), "fork");
+    launch(a, macro, kLaunchBoundary, boundary_);
+    check(cudaEventRecord(join_, boundary_), "join");
     launch(a, macro, kLaunchBulk, stream_);
     check(cudaStreamWaitEvent(stream_, join_, 0), "join");
   } else {

@@ -136,7 +136,8 @@ class Solver {
   hb_options opt_;
   Layout L_;
   cudaStream_t stream_ = nullptr;
-  cudaStream_t side_ = nullptr;   // Windkessel update and iolet records, or the boundary of an output step, beside the other sites
+  cudaStream_t side_ = nullptr;   // Windkessel update and iolet records, beside the other sites
+  cudaStream_t boundary_ = nullptr;  // the boundary of a first or output step, beside its bulk sites
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   cudaEvent_t fork_ = nullptr, join_ = nullptr;
 
