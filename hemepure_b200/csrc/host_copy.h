@@ -32,7 +32,7 @@ class HostCopy {
   // `out` as [n][width] in reference order (`order`: storage index to reference index;
   // `order_dev` the same on the device, or null: it is then uploaded once for them all).
   // A kernel reorders them, so that the host only receives them (density, velocity and
-  // stress of 4M sites: 160 ms with the reordering on the host, 12 ms so); with no device
+  // stress of 4M sites: 170 ms with the reordering on the host, 12 ms so); with no device
   // memory left for the reordered copy the host reorders it.  Fields without `out` are
   // passed over.
   struct Field {

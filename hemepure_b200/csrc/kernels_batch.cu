@@ -128,7 +128,8 @@ __device__ __forceinline__ void batch_bulk_tile(const BatchArgs& b, const MixArg
 // the SMs mix latency-bound boundary work with bandwidth-bound bulk work (the
 // assignment is static: no counter, no block-wide barrier).  The kernel is
 // latency-bound: with one site per thread it is held to 80 registers (three
-// 256-thread blocks per SM), with two to 128.
+// 256-thread blocks per SM; 72 bytes spilled in FP32, 92 in FP16), with two to 128
+// (none spilled).
 template <class S, int SPT>
 __global__ void __launch_bounds__(256, SPT == 1 ? 3 : 2) k_batch_step(const BatchArgs b) {
   const MixArgs m{b.fin, b.fout, b.gin, b.gout};
@@ -163,9 +164,9 @@ __global__ void __launch_bounds__(256, SPT == 1 ? 5 : 3) k_batch_bulk(const Batc
   batch_bulk_tile<S, SPT>(b, m, blockIdx.x);
 }
 
-// Eight blocks of 128 per SM (64 registers, ~60 bytes spilled): with the
-// batched BFL loads, ten blocks (48 registers) spilled ~160 bytes; six (80
-// registers, none spilled) measured the same as eight.  Serving probe (11
+// Eight blocks of 128 per SM (64 registers; 16 bytes spilled in FP32, 32 in FP16).
+// Before the shifted forms' present arithmetic ten blocks (48 registers) spilled ~160
+// bytes and six (80 registers, none spilled) measured the same as eight.  Serving probe (11
 // requests, 8.1M sites): 28.9k -> 30.3k MLUPS for the split step form.
 template <class S>
 __global__ void __launch_bounds__(128, 8) k_batch_gen(const BatchArgs b) {

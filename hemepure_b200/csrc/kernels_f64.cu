@@ -43,7 +43,9 @@ constexpr int kStepBlocksPerSM = 4;
 // before: 13k-site pipe 11.6 -> 7.7 us a step, 497k-site LES stenosis 44.0 -> 34.6,
 // 594k-site GZS bifurcation 105 -> 96, 4M-site pipe 213.5 -> 207.9.  Four blocks of
 // 128 (128 registers, what the BFL gather of the wall records takes) against five
-// (102): 4M-site pipe 208 / 216 us, LES stenosis 36 / 40.
+// (102): 4M-site pipe, LBGK and BFL, 208 / 216 us, LES stenosis 36 / 40.  The bound is
+// measured on BFL walls and holds for all: bounce-back and GZS forms take 118 to 128
+// registers under it, and only the sponge kernels with BFL walls spill (4 to 28 bytes).
 template <int K, int WALL>
 __global__ void __launch_bounds__(kStepBlock, kStepBlocksPerSM) k_step(const StepArgs a, const StepTiles t) {
   int b = blockIdx.x;

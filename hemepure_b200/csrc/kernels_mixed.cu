@@ -16,8 +16,10 @@
 namespace hb {
 namespace {
 
-// 64 registers.  4M-site pipe FP32: five blocks 143.5 us a step, six 128.3, seven
-// 122.7, eight 120.7; FP16: six 91, eight 85.4, ten 102.
+// 64 registers.  4M-site pipe, LBGK and BFL, FP32: five blocks 143.5 us a step, six
+// 128.3, seven 122.7, eight 120.7; FP16: six 91, eight 85.4, ten 102.  Measured on that
+// form only: bounce-back with LBGK or TRT fits, BFL spills 24 to 32 bytes, GZS 44 to 60
+// and the LES forms 56 to 92.
 constexpr int kMixedBlocksPerSM = 8;
 
 // One steady-state time step in one launch (k_step of kernels_f64.cu): boundary

@@ -486,7 +486,9 @@ int hb_setup_timing(const hb_handle* h, double ms[4]);
  * together); the next n_steps run the plain bulk sites and then the boundary
  * records, and ms[1] and ms[2] sum those. */
 int hb_profile_steps(hb_handle* h, int64_t n_steps, double ms[3]);
-/* Bytes of device memory held by the handle. */
+/* Bytes of device memory held by the handle, without the short-lived memory of
+ * set-ups and transfers: that comes from a pool of the library's own, which keeps
+ * up to 4 GB after a set-up on the device and 128 MB after a transfer. */
 int hb_device_bytes(const hb_handle* h, int64_t* bytes);
 
 #ifdef __cplusplus
